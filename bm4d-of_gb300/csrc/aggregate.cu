@@ -6,10 +6,12 @@
 // src/core/nldct.cpp:2259-2425), so each pixel's float sum follows the
 // processing order (group, then member).  Here the same sums are formed as a
 // gather with no float atomics: every member patch ("slot") is listed under
-// its origin pixel, the lists are sorted by slot number (= processing order),
-// and each pixel walks the slots that cover it in that order.  The result is
-// bit-identical to the sequential scatter.
+// the blocks of pixels it touches, each block's slots are ordered by slot
+// number (= processing order), and the block's pixels add the terms of the
+// slots that cover them in that order.  The result is bit-identical to the
+// sequential scatter.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
@@ -257,578 +259,465 @@ __global__ void count_alive_kernel(const Tile *__restrict__ tiles, int ntiles, l
 	if (ct >= 0 && total && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&counts[ct], total);
 }
 
+// places held before they are looked up and added: 512 / 1024 / 2048 took 130 /
+// 116 / 144 ms on 1920x1080x24 (barriers against resident CTAs)
+constexpr int kGatherThreads = 128, kEntCap = 1024;
+
 // ---------------------------------------------------------------------------
-// origin lists: for every tile pixel, the slots whose patch starts there,
-// sorted by slot number
+// bins: 16 x 16 pixels x BT frames of one tile (BT = 1 for one-frame patches,
+// else 4).  Every member patch ("slot") is listed in each bin it touches; a
+// CTA then adds one bin's slots to its pixels in slot order.
+//
+// The lists are small (about 2.5 entries of 4 bytes per 4x4x4 member, 2.1 per
+// 8x8 one) and their order does not matter: the gather orders a bin's slots
+// by a bitmap over the groups around it.  Aggregation with k-way merges of
+// per-pixel lists (and a weight beside every estimate) -> with bins:
+// 256x256 image, 8x8 patches 6.4 -> 0.37 ms; 767x511 colour image, defaults
+// 30.1 -> 2.1 ms; 853x481x16, defaults 35.4 -> 1.9 ms; 1920x1080x24, 4x4x4
+// patches 144 -> 114 ms.  Those merges kept 64 list heads in local memory for
+// 8x8 patches; here a slot is listed once per bin, and its terms are half the
+// bytes.
 // ---------------------------------------------------------------------------
-__global__ void list_count_kernel(long long ga, long long gb, int np, const uint8_t *__restrict__ nsimp,
-                                  const uint32_t *__restrict__ idx, const uint8_t *__restrict__ alive,
-                                  unsigned *__restrict__ cnt)
+struct BinRange {
+	int x0, x1, y0, y1, t0, t1;   // first and last bin along each axis
+};
+
+__device__ __forceinline__ BinRange bins_of(const Tile &T, const StepParams &sp, uint32_t lin)
 {
-	for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < (gb - ga) * np;
-	     it += (long long)gridDim.x * blockDim.x) {
-		const long long g = ga + it / np;
-		const int n = (int)(it % np);
-		if (!alive[g] || n >= nsimp[g]) continue;
-		atomicAdd(&cnt[idx[g * np + n]], 1u);
-	}
+	const uint32_t wh = (uint32_t)T.w * T.h;
+	const int t = (int)(lin / wh), r = (int)(lin % wh), y = r / T.w, x = r % T.w;
+	const int bt = bin_frames(sp.px, sp.pt);
+	BinRange b;
+	b.x0 = x / kBinX;
+	b.x1 = (x + sp.px - 1) / kBinX;
+	b.y0 = y / kBinY;
+	b.y1 = (y + sp.px - 1) / kBinY;
+	b.t0 = t / bt;
+	b.t1 = (t + sp.pt - 1) / bt;
+	return b;
 }
 
-__global__ void list_fill_kernel(long long ga, long long gb, int np, const uint8_t *__restrict__ nsimp,
-                                 const uint32_t *__restrict__ idx, const uint8_t *__restrict__ alive,
-                                 const unsigned *__restrict__ off, unsigned *__restrict__ cursor,
-                                 unsigned *__restrict__ list)
-{
-	for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < (gb - ga) * np;
-	     it += (long long)gridDim.x * blockDim.x) {
-		const long long g = ga + it / np;
-		const int n = (int)(it % np);
-		if (!alive[g] || n >= nsimp[g]) continue;
-		const uint32_t pos = idx[g * np + n];
-		const unsigned k = atomicAdd(&cursor[pos], 1u);
-		list[off[pos] + k] = (unsigned)it;     // chunk-relative slot number
-	}
-}
+// FILL = false: entries per bin; FILL = true: the entries, at the cursors.
+//
+// Neighbouring groups touch the same few bins, so plain atomics on the bins'
+// counters serialise (10 G entries/s on 4x4x4 patches).  A CTA therefore takes
+// kListSlots consecutive slots, counts their entries per bin in a small hash
+// table in shared memory, and takes each bin's share with one atomic.  An entry
+// that finds no place in the table (members spread over more bins than it
+// holds) goes to the global counter by itself.
+constexpr int kListThreads = 256, kListSlots = 1024, kListTable = 1024, kListProbes = 16;
 
-__global__ void list_sort_kernel(size_t npos, const unsigned *__restrict__ off, unsigned *__restrict__ list)
+template <bool FILL>
+__global__ void __launch_bounds__(kListThreads)
+bin_list_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, long long ga, long long gb,
+                const uint8_t *__restrict__ nsimp, const uint32_t *__restrict__ idx,
+                const uint8_t *__restrict__ alive, unsigned *__restrict__ cnt, unsigned *__restrict__ list)
 {
-	for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npos;
-	     p += (size_t)gridDim.x * blockDim.x) {
-		const unsigned a = off[p], b = off[p + 1];
-		for (unsigned i = a + 1; i < b; i++) {
-			const unsigned v = list[i];
-			unsigned j = i;
-			while (j > a && list[j - 1] > v) { list[j] = list[j - 1]; j--; }
-			list[j] = v;
+	__shared__ unsigned s_key[kListTable], s_cnt[kListTable];   // s_cnt: entries, then the next list place
+	const unsigned np = sp.np;
+	const long long nslots = (gb - ga) * (long long)np;
+	for (long long s0 = (long long)blockIdx.x * kListSlots; s0 < nslots; s0 += (long long)gridDim.x * kListSlots) {
+		for (int i = threadIdx.x; i < kListTable; i += kListThreads) {
+			s_key[i] = 0xffffffffu;
+			s_cnt[i] = 0u;
 		}
-	}
-}
-
-// ---------------------------------------------------------------------------
-// exclusive scan of unsigned counts (three-level, 4096 elements per block)
-// ---------------------------------------------------------------------------
-constexpr int kScanThreads = 1024, kScanPer = 4, kScanBlock = kScanThreads * kScanPer;
-
-__global__ void scan_block_kernel(unsigned *__restrict__ data, size_t n, unsigned *__restrict__ sums)
-{
-	__shared__ unsigned s[kScanThreads];
-	const size_t base = (size_t)blockIdx.x * kScanBlock + (size_t)threadIdx.x * kScanPer;
-	unsigned v[kScanPer], tot = 0;
-#pragma unroll
-	for (int i = 0; i < kScanPer; i++) {
-		v[i] = base + i < n ? data[base + i] : 0u;
-		tot += v[i];
-	}
-	s[threadIdx.x] = tot;
-	__syncthreads();
-	for (int o = 1; o < kScanThreads; o <<= 1) {
-		const unsigned add = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
 		__syncthreads();
-		s[threadIdx.x] += add;
-		__syncthreads();
-	}
-	unsigned run = s[threadIdx.x] - tot;
-#pragma unroll
-	for (int i = 0; i < kScanPer; i++) {
-		if (base + i < n) data[base + i] = run;
-		run += v[i];
-	}
-	if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = s[threadIdx.x];
-}
-
-__global__ void scan_add_kernel(unsigned *__restrict__ data, size_t n, const unsigned *__restrict__ sums)
-{
-	const size_t base = (size_t)blockIdx.x * kScanBlock;
-	const unsigned add = sums[blockIdx.x];
-	for (int i = threadIdx.x; i < kScanBlock; i += blockDim.x)
-		if (base + i < n) data[base + i] += add;
-}
-
-// ---------------------------------------------------------------------------
-// spatial lists: for every tile position (x, y, t'), the slots whose origin
-// lies in frame t' and whose patch covers (x, y), merged into slot order.
-// Entry = slot << 6 | dy << 3 | dx (dx, dy < 8 since px <= 8).
-// ---------------------------------------------------------------------------
-__global__ void slist_count_kernel(int w, int h, int F, int px, int pt, int t_lo, int t_hi,
-                                   const unsigned *__restrict__ off, unsigned *__restrict__ cnt)
-{
-	const size_t npos = (size_t)w * h * F;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < npos;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		const int x = (int)(pos % w), y = (int)((pos / w) % h), t = (int)(pos / ((size_t)w * h));
-		unsigned c = 0;
-		if (t >= t_lo && t <= t_hi && t <= F - pt)
-			for (int dy = 0; dy < px; dy++) {
-				const int oy = y - dy;
-				if (oy < 0 || oy > h - px) continue;
-				for (int dx = 0; dx < px; dx++) {
-					const int ox = x - dx;
-					if (ox < 0 || ox > w - px) continue;
-					const size_t o = ((size_t)t * h + oy) * w + ox;
-					c += off[o + 1] - off[o];
-				}
-			}
-		cnt[pos] = c;
-	}
-}
-
-// PX > 0: one list per patch offset (dy, dx), held in registers; PX == 0:
-// any patch size, lists compacted in local memory.
-template <int PX>
-__global__ void slist_build_kernel(int w, int h, int F, int px_rt, int pt, int t_lo, int t_hi,
-                                   const unsigned *__restrict__ off, const unsigned *__restrict__ list,
-                                   const unsigned *__restrict__ soff, unsigned *__restrict__ sl)
-{
-	constexpr int L = PX > 0 ? PX * PX : kMaxSpc;
-	const int px = PX > 0 ? PX : px_rt;
-	const size_t npos = (size_t)w * h * F;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < npos;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		unsigned o = soff[pos];
-		if (soff[pos + 1] == o) continue;
-		const int x = (int)(pos % w), y = (int)((pos / w) % h), t = (int)(pos / ((size_t)w * h));
-		unsigned cur[L], end[L], head[L], tag[L];
-		int nl = 0;
-#pragma unroll
-		for (int l = 0; l < L; l++) head[l] = 0xffffffffu;
-#pragma unroll
-		for (int dy = 0; dy < (PX > 0 ? PX : 8); dy++) {
-			if (dy >= px) break;
-#pragma unroll
-			for (int dx = 0; dx < (PX > 0 ? PX : 8); dx++) {
-				if (dx >= px) break;
-				const int oy = y - dy, ox = x - dx;
-				unsigned a = 0, b = 0;
-				if (oy >= 0 && oy <= h - px && ox >= 0 && ox <= w - px) {
-					const size_t q = ((size_t)t * h + oy) * w + ox;
-					a = off[q];
-					b = off[q + 1];
-				}
-				const int l = PX > 0 ? dy * PX + dx : nl;
-				if (PX > 0 || a < b) {
-					cur[l] = a; end[l] = b; tag[l] = (unsigned)(dy << 3 | dx);
-					head[l] = a < b ? list[a] : 0xffffffffu;
-					nl++;
-				}
-			}
-		}
-		// merge by slot number (slots are unique across lists)
-		for (;;) {
-			unsigned best = 0xffffffffu;
-			int bl = -1;
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if ((PX > 0 || l < nl) && head[l] < best) { best = head[l]; bl = l; }
-			if (bl < 0) break;
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if (l == bl) {
-					sl[o++] = best << 6 | tag[l];
-					head[l] = ++cur[l] < end[l] ? list[cur[l]] : 0xffffffffu;
-				}
-		}
-	}
-}
-
-// Ordered gather: each pixel merges the spatial lists of the pt origin frames
-// that cover it and adds the terms in slot order -- the order in which the
-// reference's scatter loop adds them.  PT > 0 keeps the pt list heads in
-// registers; CC is the channel count.  Each list's next entry is fetched one
-// step ahead, so that the load of the term being added and the list advance
-// overlap instead of forming one dependent chain per term.  A term's C
-// estimates and its weight term w * window[p] sit side by side in `vals`
-// (term_stride), so each term is one vector load from one 32-byte sector.
-template <int PT, int CC>
-__global__ void __launch_bounds__(128)
-gather_slist_kernel(Tile T, StepParams sp, int f_lo, int f_hi, const unsigned *__restrict__ soff,
-                    const unsigned *__restrict__ sl, const float *__restrict__ vals, float *__restrict__ acc,
-                    float *__restrict__ wacc)
-{
-	// any other pt: up to kMaxGatherPt lists (a 64-element patch of px >= 2 has
-	// at most 16 frames; runs with more patch frames are refused)
-	constexpr int L = PT > 0 ? PT : kMaxGatherPt;
-	const int px = sp.px, pt = PT > 0 ? PT : sp.pt, spc = sp.spc;
-	const size_t wh = (size_t)T.w * T.h;
-	const size_t n = wh * (size_t)(f_hi - f_lo + 1);
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-		const int t = f_lo + (int)(i / wh);
-		const size_t xy = i % wh;
-		unsigned cur[L], end[L], head[L], nxt[L];
-		bool any = false;
-#pragma unroll
-		for (int dt = 0; dt < L; dt++) {
-			head[dt] = nxt[dt] = 0xffffffffu;
-			cur[dt] = end[dt] = 0;
-			const int to = t - dt;
-			if (dt < pt && to >= 0 && to <= sp.F - pt) {
-				const size_t q = (size_t)to * wh + xy;
-				cur[dt] = soff[q];
-				end[dt] = soff[q + 1];
-				if (cur[dt] < end[dt]) {
-					head[dt] = sl[cur[dt]];
-					any = true;
-					if (cur[dt] + 1 < end[dt]) nxt[dt] = sl[cur[dt] + 1];
-				}
-			}
-		}
-		if (!any) continue;
-		const size_t pix = (size_t)t * wh + xy;
-		float a[CC];
-#pragma unroll
-		for (int c = 0; c < CC; c++) a[c] = acc[((size_t)t * CC + c) * wh + xy];
-		float wa = wacc[pix];
-		// the C estimates and the weight term of a term: one vector load
-		constexpr int TS = CC == 1 ? 2 : (CC <= 3 ? 4 : 8);
-		// terms are fetched D ahead of the one being added (a ring of D
-		// register slots, fetched and consumed in the same rotation), so that
-		// D loads of this pixel are in flight instead of one
-		constexpr int D = TS == 2 ? 8 : (TS == 4 ? 4 : 2);
-		auto fetch = [&](float (&x)[TS]) -> bool {
-			unsigned best = 0xffffffffu;
-			int bl = -1;
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if (head[l] < best) { best = head[l]; bl = l; }
-			if (bl < 0) return false;
-			const unsigned slot = best >> 6;
-			const int dx = best & 7, dy = (best >> 3) & 7;
-			const int p = (bl * px + dy) * px + dx;
-			const float *v = vals + ((size_t)slot * spc + p) * TS;
-			if (TS == 2) {
-				const float2 q = __ldg(reinterpret_cast<const float2 *>(v));
-				x[0] = q.x;
-				x[1] = q.y;
-			} else {
-#pragma unroll
-				for (int h = 0; h < TS / 4; h++) {
-					const float4 q = __ldg(reinterpret_cast<const float4 *>(v) + h);
-					x[4 * h] = q.x;
-					x[4 * h + 1] = q.y;
-					x[4 * h + 2] = q.z;
-					x[4 * h + 3] = q.w;
-				}
-			}
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if (l == bl) {
-					head[l] = nxt[l];
-					cur[l]++;
-					nxt[l] = cur[l] + 1 < end[l] ? __ldg(sl + cur[l] + 1) : 0xffffffffu;
-				}
-			return true;
-		};
-		float x[D][TS];
-		bool ok[D];
-#pragma unroll
-		for (int d = 0; d < D; d++) ok[d] = fetch(x[d]);
-		bool live = true;
-		while (live) {
-#pragma unroll
-			for (int d = 0; d < D; d++) {
-				if (live && !ok[d]) live = false;
-				if (live) {
-#pragma unroll
-					for (int c = 0; c < CC; c++) a[c] = __fadd_rn(a[c], x[d][c]);
-					wa = __fadd_rn(wa, x[d][CC]);   // w * window[p], as the reference forms it
-					ok[d] = fetch(x[d]);
-				}
-			}
-		}
-		wacc[pix] = wa;
-#pragma unroll
-		for (int c = 0; c < CC; c++) acc[((size_t)t * CC + c) * wh + xy] = a[c];
-	}
-}
-
-// ---------------------------------------------------------------------------
-// Quad path (4x4 patches): one thread per quad of 4 horizontally adjacent
-// pixels.  A member patch whose origin lies in row oy and column ox covers
-// quads (ox+3)/4 and ox/4 (one quad when ox is a multiple of 4), so a
-// quad's list holds about 7/16 of the entries of its four pixels' lists, and
-// the four pixels' terms of one member row sit in one 32-byte sector that a
-// single thread reads.  Lists are indexed by quad position
-// ((to - t_lo) * h + y) * nq + q over the chunk's origin frames [t_lo, t_hi].
-// ---------------------------------------------------------------------------
-constexpr int kQuad = 4;
-
-// row lists: for quad q, origin row oy and origin frame to, the slots whose
-// origin column lies in [4q-3, 4q+3], merged into slot order.  The origin
-// lists of consecutive columns are consecutive in `list`, so the count is one
-// difference of offsets.  Entry = slot << 3 | (ox - 4q + 3).
-__global__ void rlist_count_kernel(int w, int h, int nq, int t_lo, int nf, const unsigned *__restrict__ off,
-                                   unsigned *__restrict__ cnt)
-{
-	const size_t n = (size_t)nq * h * nf;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < n;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		const int q = (int)(pos % nq), oy = (int)((pos / nq) % h), to = t_lo + (int)(pos / ((size_t)nq * h));
-		const int lo = max(0, kQuad * q - 3), hi = min(w - kQuad, kQuad * q + 3);
-		unsigned c = 0;
-		if (oy <= h - kQuad && lo <= hi) {
-			const size_t base = ((size_t)to * h + oy) * w;
-			c = off[base + hi + 1] - off[base + lo];
-		}
-		cnt[pos] = c;
-	}
-}
-
-__global__ void rlist_build_kernel(int w, int h, int nq, int t_lo, int nf, const unsigned *__restrict__ off,
-                                   const unsigned *__restrict__ list, const unsigned *__restrict__ roff,
-                                   unsigned *__restrict__ rl)
-{
-	constexpr int L = 2 * kQuad - 1;
-	const size_t n = (size_t)nq * h * nf;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < n;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		unsigned o = roff[pos];
-		if (roff[pos + 1] == o) continue;
-		const int q = (int)(pos % nq), oy = (int)((pos / nq) % h), to = t_lo + (int)(pos / ((size_t)nq * h));
-		const size_t base = ((size_t)to * h + oy) * w;
-		unsigned cur[L], end[L], head[L];
-#pragma unroll
-		for (int l = 0; l < L; l++) {
-			const int ox = kQuad * q - 3 + l;
-			cur[l] = end[l] = 0;
-			if (ox >= 0 && ox <= w - kQuad) {
-				cur[l] = off[base + ox];
-				end[l] = off[base + ox + 1];
-			}
-			head[l] = cur[l] < end[l] ? list[cur[l]] : 0xffffffffu;
-		}
-		for (;;) {
-			unsigned best = 0xffffffffu;
-			int bl = -1;
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if (head[l] < best) { best = head[l]; bl = l; }
-			if (bl < 0) break;
-			rl[o++] = best << 3 | (unsigned)bl;
-#pragma unroll
-			for (int l = 0; l < L; l++)
-				if (l == bl) head[l] = ++cur[l] < end[l] ? list[cur[l]] : 0xffffffffu;
-		}
-	}
-}
-
-// quad lists: for quad q, pixel row y and origin frame to, the row lists of
-// origin rows y-3..y merged into slot order.  Entry = slot << 5 | dy << 3 |
-// (ox - 4q + 3), dy = y - oy.
-__global__ void qlist_count_kernel(int h, int nq, int nf, const unsigned *__restrict__ roff,
-                                   unsigned *__restrict__ cnt)
-{
-	const size_t n = (size_t)nq * h * nf;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < n;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		const int y = (int)((pos / nq) % h);
-		unsigned c = 0;
-#pragma unroll
-		for (int dy = 0; dy < kQuad; dy++) {
-			const int oy = y - dy;
-			if (oy < 0 || oy > h - kQuad) continue;
-			const size_t r = pos - (size_t)dy * nq;
-			c += roff[r + 1] - roff[r];
-		}
-		cnt[pos] = c;
-	}
-}
-
-__global__ void qlist_build_kernel(int h, int nq, int nf, const unsigned *__restrict__ roff,
-                                   const unsigned *__restrict__ rl, const unsigned *__restrict__ qoff,
-                                   unsigned *__restrict__ ql)
-{
-	const size_t n = (size_t)nq * h * nf;
-	for (size_t pos = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pos < n;
-	     pos += (size_t)gridDim.x * blockDim.x) {
-		unsigned o = qoff[pos];
-		if (qoff[pos + 1] == o) continue;
-		const int y = (int)((pos / nq) % h);
-		unsigned cur[kQuad], end[kQuad], head[kQuad];
-#pragma unroll
-		for (int dy = 0; dy < kQuad; dy++) {
-			const int oy = y - dy;
-			cur[dy] = end[dy] = 0;
-			if (oy >= 0 && oy <= h - kQuad) {
-				const size_t r = pos - (size_t)dy * nq;
-				cur[dy] = roff[r];
-				end[dy] = roff[r + 1];
-			}
-			head[dy] = cur[dy] < end[dy] ? rl[cur[dy]] : 0xffffffffu;
-		}
-		for (;;) {
-			unsigned best = 0xffffffffu;
-			int bl = -1;
-#pragma unroll
-			for (int l = 0; l < kQuad; l++)
-				if (head[l] < best) { best = head[l]; bl = l; }
-			if (bl < 0) break;
-			ql[o++] = (best >> 3) << 5 | (unsigned)bl << 3 | (best & 7u);
-#pragma unroll
-			for (int l = 0; l < kQuad; l++)
-				if (l == bl) head[l] = ++cur[l] < end[l] ? rl[cur[l]] : 0xffffffffu;
-		}
-	}
-}
-
-// Ordered gather, quad path: each thread merges the quad lists of the pt
-// origin frames covering its four pixels and adds each member's terms in
-// slot order, the order of the reference's scatter loop for every pixel.  A
-// member adds to the pixels j of the quad with 0 <= j - s < 4 (s = ox - 4q),
-// from element dx = j - s of its row.  Members are fetched D ahead of the one
-// being added (a register ring consumed in fetch order).  One member ahead
-// measured best on 1920x1080x60 (aggregation 434 ms per step against 446 ms
-// with two and 533 ms with four): fewer registers, more resident warps; the
-// batched runs' tuning may choose two (gather_depth).
-template <int PT, int CC, int D>
-__global__ void __launch_bounds__(128)
-gather_quad_kernel(Tile T, StepParams sp, int t_lo, int t_hi, int f_hi, int nq, const unsigned *__restrict__ qoff,
-                   const unsigned *__restrict__ ql, const float *__restrict__ vals, float *__restrict__ acc,
-                   float *__restrict__ wacc)
-{
-	constexpr int TS = CC == 1 ? 2 : (CC <= 3 ? 4 : 8);
-	const int w = T.w, h = T.h, spc = sp.spc;
-	const size_t wh = (size_t)w * h, plane = (size_t)nq * h;
-	const size_t n = plane * (size_t)(f_hi - t_lo + 1);
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-		const int t = t_lo + (int)(i / plane);
-		const size_t r = i % plane;
-		const int y = (int)(r / nq), q = (int)(r % nq);
-		unsigned cur[PT], end[PT], head[PT], nxt[PT];
-		bool any = false;
-#pragma unroll
-		for (int dt = 0; dt < PT; dt++) {
-			head[dt] = nxt[dt] = 0xffffffffu;
-			cur[dt] = end[dt] = 0;
-			const int to = t - dt;
-			if (to >= t_lo && to <= t_hi) {
-				const size_t qp = ((size_t)(to - t_lo) * h + y) * nq + q;
-				cur[dt] = qoff[qp];
-				end[dt] = qoff[qp + 1];
-				if (cur[dt] < end[dt]) {
-					head[dt] = __ldg(ql + cur[dt]);
-					any = true;
-					if (cur[dt] + 1 < end[dt]) nxt[dt] = __ldg(ql + cur[dt] + 1);
-				}
-			}
-		}
-		if (!any) continue;
-		const int x0 = kQuad * q;
-		const size_t pix = (size_t)t * wh + (size_t)y * w + x0;
-		float a[kQuad][CC], wa[kQuad];
-#pragma unroll
-		for (int j = 0; j < kQuad; j++) {
-			const bool in = x0 + j < w;
-#pragma unroll
-			for (int c = 0; c < CC; c++) a[j][c] = in ? acc[((size_t)t * CC + c) * wh + (size_t)y * w + x0 + j] : 0.f;
-			wa[j] = in ? wacc[pix + j] : 0.f;
-		}
-		auto fetch = [&](float (&x)[kQuad][TS], unsigned &m) -> bool {
-			unsigned best = 0xffffffffu;
-			int bl = -1;
-#pragma unroll
-			for (int l = 0; l < PT; l++)
-				if (head[l] < best) { best = head[l]; bl = l; }
-			if (bl < 0) return false;
-			const unsigned slot = best >> 5;
-			const int dy = (best >> 3) & 3, s = (int)(best & 7u) - 3;
-			const float *row = vals + ((size_t)slot * spc + (bl * kQuad + dy) * kQuad) * TS;
-			m = 0;
-#pragma unroll
-			for (int j = 0; j < kQuad; j++) {
-				const int dx = j - s;
-				if ((unsigned)dx < (unsigned)kQuad) {
-					m |= 1u << j;
-					if (TS == 2) {
-						const float2 v = __ldg(reinterpret_cast<const float2 *>(row + dx * TS));
-						x[j][0] = v.x;
-						x[j][1] = v.y;
-					} else {
-#pragma unroll
-						for (int k = 0; k < TS / 4; k++) {
-							const float4 v = __ldg(reinterpret_cast<const float4 *>(row + dx * TS) + k);
-							x[j][4 * k] = v.x;
-							x[j][4 * k + 1] = v.y;
-							x[j][4 * k + 2] = v.z;
-							x[j][4 * k + 3] = v.w;
+		for (int pass = 0; pass < (FILL ? 2 : 1); pass++) {
+			for (int k = threadIdx.x; k < kListSlots && s0 + k < nslots; k += kListThreads) {
+				const unsigned slot = (unsigned)(s0 + k);   // chunk-relative
+				const long long g = ga + slot / np;
+				const int n = (int)(slot % np);
+				if (!alive[g] || n >= nsimp[g]) continue;
+				const Tile T = tiles[tile_of(tiles, ntiles, g)];
+				const BinRange b = bins_of(T, sp, idx[g * np + n]);
+				for (int t = b.t0; t <= b.t1; t++)
+					for (int y = b.y0; y <= b.y1; y++)
+						for (int x = b.x0; x <= b.x1; x++) {
+							const unsigned bin = (unsigned)(T.bin0 + ((long long)t * T.nby + y) * T.nbx + x);
+							unsigned h = bin * 2654435761u >> 22;   // kListTable = 1024 places
+							int tries = 0;
+							for (; tries < kListProbes; tries++, h = (h + 1) & (kListTable - 1)) {
+								const unsigned key = pass ? s_key[h] : atomicCAS(&s_key[h], 0xffffffffu, bin);
+								if (key == bin || (!pass && key == 0xffffffffu)) break;
+							}
+							if (tries < kListProbes) {
+								const unsigned at = atomicAdd(&s_cnt[h], 1u);
+								if (FILL && pass) list[at] = slot;
+							} else if (FILL == (pass != 0)) {
+								const unsigned at = atomicAdd(&cnt[bin], 1u);
+								if (FILL) list[at] = slot;
+							}
 						}
+			}
+			__syncthreads();
+			if (pass == 0)
+				for (int i = threadIdx.x; i < kListTable; i += kListThreads)
+					if (s_cnt[i]) s_cnt[i] = atomicAdd(&cnt[s_key[i]], s_cnt[i]);
+			__syncthreads();
+		}
+	}
+}
+
+// List space of every bin that has entries (in any order of the bins), the
+// fill cursors, and the non-empty bins.  heads: [0] list space taken, [1]
+// non-empty bins, [2] the gather's next bin.
+__global__ void bin_alloc_kernel(unsigned nbins, const unsigned *__restrict__ cnt, unsigned *__restrict__ cursor,
+                                 unsigned *__restrict__ bins, unsigned *__restrict__ heads)
+{
+	const unsigned lane = threadIdx.x & 31u;
+	for (unsigned b0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; b0 < nbins; b0 += gridDim.x * blockDim.x) {
+		const unsigned b = b0 + lane;
+		const unsigned c = b < nbins ? cnt[b] : 0u;
+		unsigned s = c;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const unsigned u = __shfl_up_sync(0xffffffffu, s, o);
+			if (lane >= (unsigned)o) s += u;
+		}
+		const unsigned full = __ballot_sync(0xffffffffu, c != 0u);
+		if (full == 0u) continue;
+		unsigned base = 0, at = 0;
+		if (lane == 31) {
+			base = atomicAdd(&heads[0], s);
+			at = atomicAdd(&heads[1], (unsigned)__popc(full));
+		}
+		base = __shfl_sync(0xffffffffu, base, 31);
+		at = __shfl_sync(0xffffffffu, at, 31);
+		if (c) {
+			cursor[b] = base + s - c;
+			bins[at + __popc(full & ((1u << lane) - 1u))] = b;
+		}
+	}
+}
+
+// Adds a 4-row column of terms to the rows R .. R + 3 of a lane's 8 sums.  The
+// markers keep the compiler from merging the cases of R into one that indexes
+// the sums dynamically, which would put them in local memory.
+template <int R, int CC>
+__device__ __forceinline__ void add_rows(float (&a)[8][CC], float (&wa)[8], const float4 (&v)[CC], float w)
+{
+	asm volatile("" ::"n"(R));
+#pragma unroll
+	for (int h = 0; h < 4; h++)
+		if (R + h >= 0 && R + h < 8) {
+#pragma unroll
+			for (int c = 0; c < CC; c++) {
+				const float t = h == 0 ? v[c].x : h == 1 ? v[c].y : h == 2 ? v[c].z : v[c].w;
+				a[(R + h) & 7][c] = __fadd_rn(a[(R + h) & 7][c], t);
+			}
+			wa[(R + h) & 7] = __fadd_rn(wa[(R + h) & 7], w);
+		}
+	asm volatile("" ::"n"(R + 16));
+}
+
+// Ordered gather of one bin per CTA at a time.
+//
+// Order: the slots of a bin come from groups of a small box of the reference
+// grid (about 25 x 25 x 15 groups for 4x4x4 patches), and a slot's place in
+// the box -- (frame, row, column, member), row by row -- rises with its
+// number.  So the CTA marks its slots in a bitmap over the box and reads the
+// marks back in order.  A box larger than the bitmap is taken in several
+// passes, each starting at the first mark not yet taken, so any spread of the
+// members is served.
+//
+// Sums: each of the four warps owns 8 x 8 pixels x BT frames, with their sums
+// in registers, and adds a slot's terms to the pixels the slot covers, slots in
+// order: the order of the reference's scatter loop for every pixel.  Only the
+// terms a lane needs are loaded, each once; U slots' loads are in flight before
+// the first is added.  4x4 patches: a lane owns one column of 8 pixels of one
+// of four frames; the patch's four terms of that column and frame are one
+// 16-byte load (term_of orders them so), and the rows they fall on are the same
+// for the whole warp.  Other patches: a lane owns pixels (x, y) and (x, y + 4).
+template <int PX, int BT, int CC, int U>
+__global__ void __launch_bounds__(kGatherThreads)
+bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, long long ga,
+                  const uint32_t *__restrict__ idx, const float *__restrict__ vals, const float *__restrict__ wslot,
+                  const float *__restrict__ win, const unsigned *__restrict__ cnt,
+                  const unsigned *__restrict__ cursor, const unsigned *__restrict__ bins, unsigned *__restrict__ heads,
+                  const unsigned *__restrict__ list, float *__restrict__ acc, float *__restrict__ wacc)
+{
+	constexpr int kBitWords = BT == 1 ? 512 : 2048;
+	constexpr bool kColumn = PX == 4;
+	static_assert(!kColumn || BT == 4, "a lane's frame is one of four");
+	__shared__ unsigned s_bits[kBitWords];
+	__shared__ uint4 s_ent[kEntCap];         // slot, place relative to the bin, weight
+	__shared__ float s_win[64];
+	__shared__ unsigned s_warp[2][kGatherThreads / 32];
+	__shared__ int s_box[6];
+	__shared__ unsigned s_bin;
+	__shared__ unsigned long long s_next;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int px = PX ? PX : sp.px, pt = sp.pt, np = sp.np, spc = px * px * pt;
+	const unsigned nfull = heads[1];
+	for (int i = tid; i < px * px; i += kGatherThreads) s_win[i] = win[i];
+	for (;;) {
+		__syncthreads();
+		if (tid == 0) s_bin = atomicAdd(&heads[2], 1u);
+		if (tid < 6) s_box[tid] = (tid & 1) ? -1 : 0x7fffffff;
+		__syncthreads();
+		if (s_bin >= nfull) break;
+		const unsigned bin = bins[s_bin];
+		int ti = 0;
+		while (ti + 1 < ntiles && tiles[ti + 1].bin0 <= (long long)bin) ti++;
+		const Tile T = tiles[ti];
+		const int lb = (int)((long long)bin - T.bin0);
+		const int X0 = lb % T.nbx * kBinX, Y0 = lb / T.nbx % T.nby * kBinY, F0 = lb / (T.nbx * T.nby) * BT;
+		const unsigned n = cnt[bin];
+		const unsigned *lst = list + (cursor[bin] - n);   // the cursor stands past the last entry
+		const unsigned l0 = (unsigned)(ga - T.g0);        // of the tile's first group in the chunk (may wrap)
+		const unsigned wh = (unsigned)T.w * T.h;
+		const unsigned nx = T.nx, ny = T.ny;
+
+		// the box of groups
+		{
+			int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
+			for (unsigned i = tid; i < n; i += kGatherThreads) {
+				const unsigned l = l0 + lst[i] / np, r = l / nx;
+				const int v[3] = {(int)(l % nx), (int)(r % ny), (int)(r / ny)};
+#pragma unroll
+				for (int k = 0; k < 3; k++) { lo[k] = min(lo[k], v[k]); hi[k] = max(hi[k], v[k]); }
+			}
+#pragma unroll
+			for (int k = 0; k < 3; k++) {
+				lo[k] = __reduce_min_sync(0xffffffffu, lo[k]);
+				hi[k] = __reduce_max_sync(0xffffffffu, hi[k]);
+				if (lane == 0) { atomicMin(&s_box[2 * k], lo[k]); atomicMax(&s_box[2 * k + 1], hi[k]); }
+			}
+		}
+		__syncthreads();
+		const int gx0 = s_box[0], gy0 = s_box[2], gt0 = s_box[4];
+		const unsigned bnx = (unsigned)(s_box[1] - gx0 + 1), bny = (unsigned)(s_box[3] - gy0 + 1);
+		const unsigned long long volume = (unsigned long long)(s_box[5] - gt0 + 1) * bny * bnx * np;
+		auto place = [&](unsigned slot) -> unsigned long long {
+			const unsigned q = slot / np, l = l0 + q, r = l / nx;
+			const unsigned x = l % nx - gx0, y = r % ny - gy0, t = r / ny - gt0;
+			return ((unsigned long long)(t * bny + y) * bnx + x) * np + (slot - q * np);
+		};
+
+		// this warp's pixels; sum s of a lane is pixel (x, ly(s)) of frame lf(s)
+		const int qx = X0 + (warp & 1) * 8, qy = Y0 + (warp >> 1) * 8;
+		const int x = qx + (lane & 7), y = qy + (lane >> 3);
+		constexpr int NS = kColumn ? 8 : 2 * BT;
+		auto ly = [&](int s) { return kColumn ? qy + s : y + 4 * (s & 1); };
+		auto lf = [&](int s) { return kColumn ? F0 + (lane >> 3) : F0 + (s >> 1); };
+		float a[NS][CC], wa[NS];
+#pragma unroll
+		for (int s = 0; s < NS; s++) {
+			const bool in = x < T.w && ly(s) < T.h && lf(s) < sp.F;
+			const size_t at = (size_t)ly(s) * T.w + x;
+#pragma unroll
+			for (int c = 0; c < CC; c++) a[s][c] = in ? acc[T.pix0 * CC + ((size_t)lf(s) * CC + c) * wh + at] : 0.f;
+			wa[s] = in ? wacc[T.pix0 + (size_t)lf(s) * wh + at] : 0.f;
+		}
+
+		unsigned long long p0 = 0;
+		for (;;) {
+			// marks of the slots at places [p0, p0 + bits)
+			for (int i = tid; i < kBitWords; i += kGatherThreads) s_bits[i] = 0u;
+			if (tid == 0) s_next = ~0ull;
+			__syncthreads();
+			unsigned long long nxt = ~0ull;
+			for (unsigned i = tid; i < n; i += kGatherThreads) {
+				const unsigned long long p = place(lst[i]);
+				if (p < p0) continue;
+				if (p - p0 < (unsigned long long)kBitWords * 32u) atomicOr(&s_bits[(unsigned)(p - p0) >> 5], 1u << ((unsigned)(p - p0) & 31u));
+				else nxt = p < nxt ? p : nxt;
+			}
+			if (nxt != ~0ull) atomicMin(&s_next, nxt);
+			__syncthreads();
+			const unsigned q0 = (unsigned)(p0 / np), m0 = (unsigned)(p0 - (unsigned long long)q0 * np);
+			const int words = (int)min((unsigned long long)kBitWords, (volume - p0 + 31) / 32);
+			// the marks in order, one word per thread and round; the places found
+			// gather in s_ent until it is full (or the words run out)
+			unsigned have = 0;
+			for (int w0 = 0, odd = 0;; w0 += kGatherThreads, odd ^= 1) {
+				const bool last = w0 >= words;
+				unsigned bits = last ? 0u : s_bits[w0 + tid], rank = 0, total = 0;
+				if (!last) {
+					const unsigned c = __popc(bits);
+					unsigned s = c;
+#pragma unroll
+					for (int o = 1; o < 32; o <<= 1) {
+						const unsigned u = __shfl_up_sync(0xffffffffu, s, o);
+						if (lane >= o) s += u;
+					}
+					if (lane == 31) s_warp[odd][warp] = s;
+					__syncthreads();
+					rank = s - c;
+#pragma unroll
+					for (int k = 0; k < kGatherThreads / 32; k++) {
+						if (k < warp) rank += s_warp[odd][k];
+						total += s_warp[odd][k];
 					}
 				}
-			}
-#pragma unroll
-			for (int l = 0; l < PT; l++)
-				if (l == bl) {
-					head[l] = nxt[l];
-					cur[l]++;
-					nxt[l] = cur[l] + 1 < end[l] ? __ldg(ql + cur[l] + 1) : 0xffffffffu;
-				}
-			return true;
-		};
-		float x[D][kQuad][TS];
-		unsigned m[D];
-		bool ok[D];
-#pragma unroll
-		for (int d = 0; d < D; d++) ok[d] = fetch(x[d], m[d]);
-		bool live = true;
-		while (live) {
-#pragma unroll
-			for (int d = 0; d < D; d++) {
-				if (live && !ok[d]) live = false;
-				if (live) {
-#pragma unroll
-					for (int j = 0; j < kQuad; j++)
-						if (m[d] >> j & 1u) {
-#pragma unroll
-							for (int c = 0; c < CC; c++) a[j][c] = __fadd_rn(a[j][c], x[d][j][c]);
-							wa[j] = __fadd_rn(wa[j], x[d][j][CC]);   // w * window[p], as the reference forms it
+				unsigned done = 0;
+				while (done < total || (last && have)) {
+					const unsigned room = (unsigned)kEntCap - have;
+					while (bits && rank - done < room) {
+						const int b = __ffs(bits) - 1;
+						bits &= bits - 1;
+						s_ent[have + rank - done].x = (unsigned)((w0 + tid) * 32 + b);
+						rank++;
+					}
+					const unsigned put = min(room, total - done);
+					have += put;
+					done += put;
+					if (have < (unsigned)kEntCap && !last) continue;
+					const int ne = (int)have;
+					have = 0;
+					__syncthreads();
+					for (int e = tid; e < ne; e += kGatherThreads) {
+						const unsigned p = m0 + s_ent[e].x, qq = p / np, m = p - qq * np, q = q0 + qq;
+						const unsigned gx = q % bnx + gx0, r = q / bnx, gy = r % bny + gy0, gt = r / bny + gt0;
+						const unsigned slot = ((gt * ny + gy) * nx + gx - l0) * np + m;
+						const unsigned lin = __ldg(idx + (size_t)ga * np + slot);
+						const int ot = (int)(lin / wh), rr = (int)(lin % wh), oy = rr / T.w, ox = rr % T.w;
+						s_ent[e] = make_uint4(slot, (unsigned)(ox - X0 + 8) | (unsigned)(oy - Y0 + 8) << 8 |
+						                                (unsigned)(ot - F0 + 16) << 16,
+						                      __float_as_uint(__ldg(wslot + slot)), 0u);
+					}
+					__syncthreads();
+					for (int e = 0; e < ne; e += 32) {
+						bool hit = false;
+						if (e + lane < ne) {
+							const unsigned pos = s_ent[e + lane].y;
+							const int rx = (int)(pos & 255u) - 8 + X0 - qx, ry = (int)(pos >> 8 & 255u) - 8 + Y0 - qy;
+							hit = rx < 8 && rx + px > 0 && ry < 8 && ry + px > 0;
 						}
-					ok[d] = fetch(x[d], m[d]);
+						unsigned m = __ballot_sync(0xffffffffu, hit);
+						if constexpr (kColumn) {
+							while (m) {
+								float4 v[U][CC];
+								float wt[U];
+								int row[U];
+								bool ok[U];
+#pragma unroll
+								for (int u = 0; u < U; u++) {
+									row[u] = -4;
+									ok[u] = false;
+									if (!m) continue;
+									const uint4 q = s_ent[e + __ffs(m) - 1];
+									m &= m - 1;
+									const unsigned dx = (unsigned)(x - X0 + 8) - (q.y & 255u);
+									const unsigned dt = (unsigned)((lane >> 3) + 16) - (q.y >> 16);
+									row[u] = (int)(q.y >> 8 & 255u) - 8 + Y0 - qy;
+									ok[u] = dx < 4u && dt < (unsigned)pt;
+									wt[u] = __uint_as_float(q.z);   // no window for these patches
+									const float *col = vals + (size_t)q.x * (spc * CC) + (dt * 4u + dx) * 4u;
+#pragma unroll
+									for (int c = 0; c < CC; c++)
+										if (ok[u]) v[u][c] = __ldg(reinterpret_cast<const float4 *>(col + c * spc));
+								}
+#pragma unroll
+								for (int u = 0; u < U; u++)
+									if (ok[u]) {
+										switch (row[u]) {   // the same for the whole warp
+										case -3: add_rows<-3>(a, wa, v[u], wt[u]); break;
+										case -2: add_rows<-2>(a, wa, v[u], wt[u]); break;
+										case -1: add_rows<-1>(a, wa, v[u], wt[u]); break;
+										case 0: add_rows<0>(a, wa, v[u], wt[u]); break;
+										case 1: add_rows<1>(a, wa, v[u], wt[u]); break;
+										case 2: add_rows<2>(a, wa, v[u], wt[u]); break;
+										case 3: add_rows<3>(a, wa, v[u], wt[u]); break;
+										case 4: add_rows<4>(a, wa, v[u], wt[u]); break;
+										case 5: add_rows<5>(a, wa, v[u], wt[u]); break;
+										case 6: add_rows<6>(a, wa, v[u], wt[u]); break;
+										case 7: add_rows<7>(a, wa, v[u], wt[u]); break;
+										}
+									}
+							}
+						} else {
+							while (m) {
+								float v[U][NS][CC], wt[U][2];
+								unsigned fm[U];
+								bool ok[U][2];
+#pragma unroll
+								for (int u = 0; u < U; u++) {
+									fm[u] = 0u;
+									ok[u][0] = ok[u][1] = false;
+									if (!m) continue;
+									const uint4 q = s_ent[e + __ffs(m) - 1];
+									m &= m - 1;
+									const int dx = x - X0 + 8 - (int)(q.y & 255u), dy = y - Y0 + 8 - (int)(q.y >> 8 & 255u);
+									const int rt = (int)(q.y >> 16) - 16;
+									const bool okx = (unsigned)dx < (unsigned)px;
+									ok[u][0] = okx && (unsigned)dy < (unsigned)px;
+									ok[u][1] = okx && (unsigned)(dy + 4) < (unsigned)px;
+									const float *row = vals + (size_t)q.x * (spc * CC);
+#pragma unroll
+									for (int h = 0; h < 2; h++) {
+										const int d = (dy + 4 * h) * px + dx;
+										// as the reference forms it
+										wt[u][h] = ok[u][h] ? __fmul_rn(__uint_as_float(q.z), s_win[d]) : 0.f;
+#pragma unroll
+										for (int f = 0; f < BT; f++) {
+											const int dt = f - rt;
+											if ((unsigned)dt >= (unsigned)pt) continue;
+											fm[u] |= 1u << f;
+#pragma unroll
+											for (int c = 0; c < CC; c++)
+												if (ok[u][h]) v[u][2 * f + h][c] = __ldg(row + (c * spc + dt * px * px + d));
+										}
+									}
+								}
+#pragma unroll
+								for (int u = 0; u < U; u++)
+#pragma unroll
+									for (int s = 0; s < NS; s++)
+										if ((fm[u] >> (s >> 1) & 1u) && ok[u][s & 1]) {
+#pragma unroll
+											for (int c = 0; c < CC; c++) a[s][c] = __fadd_rn(a[s][c], v[u][s][c]);
+											wa[s] = __fadd_rn(wa[s], wt[u][s & 1]);
+										}
+							}
+						}
+					}
+					__syncthreads();
 				}
+				if (last) break;
 			}
+			p0 = s_next;
+			__syncthreads();
+			if (p0 == ~0ull) break;
 		}
 #pragma unroll
-		for (int j = 0; j < kQuad; j++)
-			if (x0 + j < w) {
+		for (int s = 0; s < NS; s++) {
+			if (!(x < T.w && ly(s) < T.h && lf(s) < sp.F)) continue;
+			const size_t at = (size_t)ly(s) * T.w + x;
 #pragma unroll
-				for (int c = 0; c < CC; c++) acc[((size_t)t * CC + c) * wh + (size_t)y * w + x0 + j] = a[j][c];
-				wacc[pix + j] = wa[j];
-			}
+			for (int c = 0; c < CC; c++) acc[T.pix0 * CC + ((size_t)lf(s) * CC + c) * wh + at] = a[s][c];
+			wacc[T.pix0 + (size_t)lf(s) * wh + at] = wa[s];
+		}
 	}
 }
 
-template <int CC, int D>
-void gather_quad_d(int gb, cudaStream_t st, const Tile &T, const StepParams &sp, int t_lo, int t_hi, int f_hi,
-                   int nq, const unsigned *qoff, const unsigned *ql, const float *vals, float *acc, float *wacc)
+template <int PX, int BT, int CC, int U>
+cudaError_t gather_t(const BinArgs &a, const Tile *tiles, int ntiles, const StepParams &sp, long long ga,
+                     const uint32_t *idx, const float *vals, const float *wslot, const float *win, float *acc,
+                     float *wacc, int nsm, cudaStream_t st)
 {
-	switch (sp.pt) {
-	case 1:
-		gather_quad_kernel<1, CC, D><<<gb, 128, 0, st>>>(T, sp, t_lo, t_hi, f_hi, nq, qoff, ql, vals, acc, wacc);
-		break;
-	case 2:
-		gather_quad_kernel<2, CC, D><<<gb, 128, 0, st>>>(T, sp, t_lo, t_hi, f_hi, nq, qoff, ql, vals, acc, wacc);
-		break;
-	default:
-		gather_quad_kernel<4, CC, D><<<gb, 128, 0, st>>>(T, sp, t_lo, t_hi, f_hi, nq, qoff, ql, vals, acc, wacc);
-		break;
-	}
+	auto kern = bin_gather_kernel<PX, BT, CC, U>;
+	int per_sm = 0;
+	cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGatherThreads, 0);
+	if (e != cudaSuccess) return e;
+	const long long blocks = std::min<long long>((long long)nsm * std::max(per_sm, 1), a.nbins);
+	kern<<<(int)blocks, kGatherThreads, 0, st>>>(tiles, ntiles, sp, ga, idx, vals, wslot, win, a.cnt, a.cursor, a.bins,
+	                                            a.heads, a.list, acc, wacc);
+	return cudaGetLastError();
 }
 
-template <int CC>
-void gather_quad_pt(int gb, cudaStream_t st, const Tile &T, const StepParams &sp, int t_lo, int t_hi, int f_hi,
-                    int nq, const unsigned *qoff, const unsigned *ql, const float *vals, float *acc, float *wacc)
+// Slots whose loads are in flight: 4x4 patches take one 16-byte load per
+// channel (2 / 4 slots: 117 / 114 ms of aggregation on 1920x1080x24, 16.2 /
+// 14.7 ms on 640x360x3x14; 8 by gather_depth 2), the others one or two 4-byte
+// loads per frame and channel.
+template <int CC, class... Args>
+cudaError_t gather_c(const StepParams &sp, Args... args)
 {
-	if (sp.gather_depth == 2) gather_quad_d<CC, 2>(gb, st, T, sp, t_lo, t_hi, f_hi, nq, qoff, ql, vals, acc, wacc);
-	else gather_quad_d<CC, 1>(gb, st, T, sp, t_lo, t_hi, f_hi, nq, qoff, ql, vals, acc, wacc);
-}
-
-template <int CC>
-void gather_pt(int gb, cudaStream_t st, const Tile &T, const StepParams &sp, int t_lo, int f_hi,
-               const unsigned *soff, const unsigned *sl, const float *vals, float *acc, float *wacc)
-{
-	switch (sp.pt) {
-	case 1: gather_slist_kernel<1, CC><<<gb, 128, 0, st>>>(T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc); break;
-	case 2: gather_slist_kernel<2, CC><<<gb, 128, 0, st>>>(T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc); break;
-	case 4: gather_slist_kernel<4, CC><<<gb, 128, 0, st>>>(T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc); break;
-	default: gather_slist_kernel<0, CC><<<gb, 128, 0, st>>>(T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc); break;
-	}
+	if (sp.px == 4) return sp.gather_depth == 2 && CC == 1 ? gather_t<4, 4, CC, CC == 1 ? 8 : 4>(args...) : gather_t<4, 4, CC, 4>(args...);
+	if (sp.pt != 1) return gather_t<0, 4, CC, 1>(args...);
+	if (sp.px == 7) return gather_t<7, 1, CC, CC == 1 ? 4 : 2>(args...);
+	if (sp.px == 8) return gather_t<8, 1, CC, CC == 1 ? 4 : 2>(args...);
+	return gather_t<0, 1, CC, 2>(args...);
 }
 
 // ---------------------------------------------------------------------------
@@ -971,104 +860,30 @@ cudaError_t launch_count_alive(const Tile *tiles, int ntiles, long long G, const
 	return cudaGetLastError();
 }
 
-// Kernels exclusive_scan launches for n entries.
-unsigned scan_kernels(size_t n)
+int bin_entries_per_member(const StepParams &sp)
 {
-	const size_t nb = (n + 1 + kScanBlock - 1) / kScanBlock;
-	return nb > 1 ? 2 + scan_kernels(nb - 1) : 1;
+	const int bt = bin_frames(sp.px, sp.pt), s = sp.px > 1 ? 2 : 1;
+	return s * s * ((sp.pt + bt - 2) / bt + 1);
 }
 
-// Exclusive scan of data[0..n) in place; data[n] receives the total.
-cudaError_t exclusive_scan(unsigned *data, size_t n, unsigned *scratch, cudaStream_t st)
+cudaError_t launch_aggregate(const BinArgs &a, const Tile *tiles, int ntiles, const StepParams &sp, long long ga,
+                             long long gb, const uint8_t *nsimp, const uint32_t *idx, const uint8_t *alive,
+                             const float *vals, const float *wslot, const float *win, float *acc, float *wacc, int nsm,
+                             unsigned *launches, cudaStream_t st)
 {
-	// data must hold n+1 entries; scratch needs ceil(n/4096) + ceil(n/4096^2) + 2 entries
-	const size_t nb = (n + 1 + kScanBlock - 1) / kScanBlock;
-	scan_block_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(data, n + 1, scratch);
-	if (nb > 1) {
-		cudaError_t e = exclusive_scan(scratch, nb - 1, scratch + nb + 1, st);
-		if (e != cudaSuccess) return e;
-		scan_add_kernel<<<(unsigned)nb, 256, 0, st>>>(data, n + 1, scratch);
-	}
-	return cudaGetLastError();
-}
-
-cudaError_t launch_lists(long long ga, long long gb, int np, const uint8_t *nsimp, const uint32_t *idx,
-                         const uint8_t *alive, size_t npos, unsigned *cnt, unsigned *off, unsigned *list,
-                         unsigned *scratch, unsigned *launches, cudaStream_t st)
-{
-	*launches += 3 + scan_kernels(npos);
-	cudaError_t e = cudaMemsetAsync(off, 0, (npos + 1) * sizeof(unsigned), st);
+	if (gb <= ga || a.nbins == 0) return cudaSuccess;
+	*launches += 4;
+	cudaError_t e = cudaMemsetAsync(a.heads, 0, sizeof(unsigned) * (kBinHeads + (size_t)a.nbins), st);   // heads, cnt
 	if (e != cudaSuccess) return e;
-	const long long ns = (gb - ga) * np;
-	list_count_kernel<<<grid_for(ns, 256, 16384), 256, 0, st>>>(ga, gb, np, nsimp, idx, alive, off);
-	e = exclusive_scan(off, npos, scratch, st);
+	const int lb = grid_for((gb - ga) * sp.np, kListSlots, 16384);
+	bin_list_kernel<false><<<lb, kListThreads, 0, st>>>(tiles, ntiles, sp, ga, gb, nsimp, idx, alive, a.cnt, nullptr);
+	bin_alloc_kernel<<<grid_for(a.nbins, 256, 4096), 256, 0, st>>>(a.nbins, a.cnt, a.cursor, a.bins, a.heads);
+	bin_list_kernel<true><<<lb, kListThreads, 0, st>>>(tiles, ntiles, sp, ga, gb, nsimp, idx, alive, a.cursor, a.list);
+	e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
-	e = cudaMemsetAsync(cnt, 0, npos * sizeof(unsigned), st);
-	if (e != cudaSuccess) return e;
-	list_fill_kernel<<<grid_for(ns, 256, 16384), 256, 0, st>>>(ga, gb, np, nsimp, idx, alive, off, cnt, list);
-	list_sort_kernel<<<grid_for((long long)npos, 256, 16384), 256, 0, st>>>(npos, off, list);
-	return cudaGetLastError();
-}
-
-bool quad_path(const StepParams &sp)
-{
-	return sp.px == kQuad && (sp.pt == 1 || sp.pt == 2 || sp.pt == 4);
-}
-
-int list_entries_per_member(const StepParams &sp)
-{
-	// quad path: at most 2 row-list and 8 quad-list entries per member
-	return quad_path(sp) ? 10 : sp.px * sp.px;
-}
-
-cudaError_t launch_gather(const Tile &T, const StepParams &sp, int t_lo, int t_hi, const unsigned *off,
-                          const unsigned *list, unsigned *cnt, unsigned *soff, unsigned *sl, size_t members,
-                          unsigned *scratch, const float *vals, float *acc, float *wacc, unsigned *launches,
-                          cudaStream_t st)
-{
-	// origin frames [t_lo, t_hi] hold the chunk's member patches; pixels of
-	// frames [t_lo, t_hi + pt - 1] receive them
-	if (t_hi < t_lo) return cudaSuccess;
-	const int f_hi = t_hi + sp.pt - 1 < sp.F - 1 ? t_hi + sp.pt - 1 : sp.F - 1;
-	if (quad_path(sp)) {
-		// row-list offsets in cnt (free once the origin lists are sorted), row
-		// lists then quad lists in sl
-		const int nq = (T.w + kQuad - 1) / kQuad, nf = t_hi - t_lo + 1;
-		const size_t nqp = (size_t)nq * T.h * nf;
-		const int b = grid_for((long long)nqp, 256, 16384);
-		unsigned *roff = cnt, *rl = sl, *ql = sl + 2 * members;
-		*launches += 5 + 2 * scan_kernels(nqp);
-		rlist_count_kernel<<<b, 256, 0, st>>>(T.w, T.h, nq, t_lo, nf, off, roff);
-		cudaError_t e = exclusive_scan(roff, nqp, scratch, st);
-		if (e != cudaSuccess) return e;
-		rlist_build_kernel<<<b, 256, 0, st>>>(T.w, T.h, nq, t_lo, nf, off, list, roff, rl);
-		qlist_count_kernel<<<b, 256, 0, st>>>(T.h, nq, nf, roff, soff);
-		e = exclusive_scan(soff, nqp, scratch, st);
-		if (e != cudaSuccess) return e;
-		qlist_build_kernel<<<b, 256, 0, st>>>(T.h, nq, nf, roff, rl, soff, ql);
-		const long long nthr = (long long)nq * T.h * (f_hi - t_lo + 1);
-		const int gb = grid_for(nthr, 128, 65535);
-		if (sp.C == 1) gather_quad_pt<1>(gb, st, T, sp, t_lo, t_hi, f_hi, nq, soff, ql, vals, acc, wacc);
-		else if (sp.C == 3) gather_quad_pt<3>(gb, st, T, sp, t_lo, t_hi, f_hi, nq, soff, ql, vals, acc, wacc);
-		else gather_quad_pt<4>(gb, st, T, sp, t_lo, t_hi, f_hi, nq, soff, ql, vals, acc, wacc);
-		return cudaGetLastError();
-	}
-	const size_t npos = (size_t)T.w * T.h * sp.F;
-	const int b = grid_for((long long)npos, 256, 16384);
-	*launches += 3 + scan_kernels(npos);
-	slist_count_kernel<<<b, 256, 0, st>>>(T.w, T.h, sp.F, sp.px, sp.pt, t_lo, t_hi, off, soff);
-	cudaError_t e = exclusive_scan(soff, npos, scratch, st);
-	if (e != cudaSuccess) return e;
-	if (sp.px == 4)
-		slist_build_kernel<4><<<b, 256, 0, st>>>(T.w, T.h, sp.F, sp.px, sp.pt, t_lo, t_hi, off, list, soff, sl);
-	else
-		slist_build_kernel<0><<<b, 256, 0, st>>>(T.w, T.h, sp.F, sp.px, sp.pt, t_lo, t_hi, off, list, soff, sl);
-	const long long npix = (long long)T.w * T.h * (f_hi - t_lo + 1);
-	const int gb = grid_for(npix, 128, 65535);
-	if (sp.C == 1) gather_pt<1>(gb, st, T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc);
-	else if (sp.C == 3) gather_pt<3>(gb, st, T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc);
-	else gather_pt<4>(gb, st, T, sp, t_lo, f_hi, soff, sl, vals, acc, wacc);
-	return cudaGetLastError();
+	if (sp.C == 1) return gather_c<1>(sp, a, tiles, ntiles, sp, ga, idx, vals, wslot, win, acc, wacc, nsm, st);
+	if (sp.C == 3) return gather_c<3>(sp, a, tiles, ntiles, sp, ga, idx, vals, wslot, win, acc, wacc, nsm, st);
+	return gather_c<4>(sp, a, tiles, ntiles, sp, ga, idx, vals, wslot, win, acc, wacc, nsm, st);
 }
 
 cudaError_t launch_color(const Image &in, const Image &out, int forward, cudaStream_t st)

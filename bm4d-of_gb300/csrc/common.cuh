@@ -36,7 +36,8 @@ struct Tile {                     // one spatial tile (crop) of one step
 	int gx, gy, gf;               // offsets of the grid coordinate lists
 	long long g0;                 // first group id of this tile
 	long long pix0;               // first pixel of this tile's aggregation buffers
-	unsigned long long lin0;      // first origin-list slot (== pix0)
+	long long bin0;               // first aggregation bin of this tile
+	int nbx, nby;                 // its bins along x and y
 	int bx0, by0, bx1, by1;       // crop touches an inner border (nldct.cpp:520-525)
 };
 
@@ -52,7 +53,7 @@ struct StepParams {               // resolved parameters of one step
 	float beta1;                  // learned form: hard threshold of the non-mean Haar rows
 	int search_ctas;              // exact search: CTAs per SM (4 or 6; 0 = default)
 	int search_strip;             // exact search: candidates per thread along a column (7 or 21; 0 = default)
-	int gather_depth;             // quad gather: members in flight per thread (1 or 2; 0 = 1)
+	int gather_depth;             // ordered gather: staging depth (1 or 2; 0 = 1)
 	float beta_mean;              // betaMean (order-invariant filtering)
 	int order_inv;                // orderInvariance
 	int vbm3d;                    // predictive search (the reference's VBM3D_SEARCH build)
@@ -62,11 +63,19 @@ struct StepParams {               // resolved parameters of one step
 };
 
 // Aggregation terms of a chunk of groups: for slot s (one member of one
-// group) and patch element p, the C weighted estimates (w * window[p]) * ghat
-// followed by the weight term w * window[p], so that the ordered gather reads
-// one aligned vector per term:  vals[(s * spc + p) * term_stride(C) + c],
-// c = 0..C (c = C: the weight term).
-__host__ __device__ __forceinline__ int term_stride(int C) { return C == 1 ? 2 : (C <= 3 ? 4 : 8); }
+// group), channel c and patch element p, the weighted estimate
+// (w * window[p]) * ghat at vals[(s * C + c) * spc + term_of(px, p)], and the
+// member's weight w at wslot[s] (the gather forms w * window[p] itself).  4x4
+// patches hold each frame's elements column by column, so that the gather's
+// lanes read the four rows of a column with one load.
+__host__ __device__ __forceinline__ int term_of(int px, int p)
+{
+	return px == 4 ? (p & ~15) | (p & 3) << 2 | (p >> 2 & 3) : p;
+}
+
+// Aggregation bins: pixels x frames of one tile.
+constexpr int kBinX = 16, kBinY = 16;
+__host__ __device__ __forceinline__ int bin_frames(int px, int pt) { return pt == 1 && px != 4 ? 1 : 4; }
 
 // Locate the tile owning global group g (tiles are few: linear scan).
 __device__ __forceinline__ int tile_of(const Tile *tiles, int ntiles, long long g)

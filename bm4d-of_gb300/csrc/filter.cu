@@ -166,7 +166,7 @@ filter_exact_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, in
                     const float *__restrict__ win, long long g_begin, long long g_end,
                     const uint8_t *__restrict__ nsimp, const uint32_t *__restrict__ idx,
                     const uint8_t *__restrict__ alive, float *__restrict__ vals,
-                    float *__restrict__ wgroup, uint8_t *__restrict__ eq)
+                    float *__restrict__ wslot, float *__restrict__ wgroup, uint8_t *__restrict__ eq)
 {
 	extern __shared__ __align__(16) float sm[];
 	const int px = PX ? PX : sp.px, pt = PT ? PT : sp.pt, C = CC ? CC : sp.C;
@@ -245,13 +245,12 @@ filter_exact_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, in
 				for (int n = 1; n < ns; n++) differs |= row[n] != row[0];
 			}
 		const int any = __syncthreads_or(differs);
-		const int ts = term_stride(C);
 		if (ns > 1 && !any) {
 			// unweighted: the weights are set later (fixup_equal_kernel)
 			for (int it = tid; it < ns * per; it += blockDim.x) {
 				const int n = it / per, r = it % per;
 				const int c = r / spc, p = r % spc;
-				vals[((slot0 + n) * spc + p) * ts + c] = Gn[r * nsp + n];
+				vals[((slot0 + n) * C + c) * spc + term_of(px, p)] = Gn[r * nsp + n];
 			}
 			if (tid == 0) eq[g] = 1;
 			continue;
@@ -315,12 +314,9 @@ filter_exact_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, in
 		for (int it = tid; it < ns * per; it += blockDim.x) {
 			const int n = it / per, r = it % per;
 			const int c = r / spc, p = r % spc;
-			vals[((slot0 + n) * spc + p) * ts + c] = __fmul_rn(__fmul_rn(w, wn[p]), Gn[r * nsp + n]);
+			vals[((slot0 + n) * C + c) * spc + term_of(px, p)] = __fmul_rn(__fmul_rn(w, wn[p]), Gn[r * nsp + n]);
 		}
-		for (int it = tid; it < ns * spc; it += blockDim.x) {
-			const int n = it / spc, p = it % spc;
-			vals[((slot0 + n) * spc + p) * ts + C] = __fmul_rn(w, wn[p]);
-		}
+		if (tid < ns) wslot[slot0 + tid] = w;
 		if (tid == 0) { wgroup[g] = w; eq[g] = 0; }
 	}
 }
@@ -391,7 +387,7 @@ filter_quad_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, int
                    const float *__restrict__ basis, const float *__restrict__ binv, const float *__restrict__ win,
                    long long g_begin, long long g_end, const uint8_t *__restrict__ nsimp,
                    const uint32_t *__restrict__ idx, const uint8_t *__restrict__ alive, float *__restrict__ vals,
-                   float *__restrict__ wgroup, uint8_t *__restrict__ eq)
+                   float *__restrict__ wslot, float *__restrict__ wgroup, uint8_t *__restrict__ eq)
 {
 	constexpr int SPC = PX * PX * PT;
 	static_assert(SPC == 64, "four-group filter: 64-element patches");
@@ -428,7 +424,7 @@ filter_quad_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, int
 	const bool oinv = sp.order_inv != 0;
 	const float is2 = (float)(1.0 / sqrt(2.0));
 	const int bar = 1 + sub, lane = t & 31, w = t >> 5;
-	const int ht = t / (PX * PX), hy = (t / PX) % PX, hx = t % PX;
+	const int ht = t / (PX * PX), hy = (t / PX) % PX, hx = t % PX, at = term_of(PX, t);
 
 	for (long long g = g_begin + (long long)blockIdx.x * kQuadGroups + sub; g < g_end;
 	     g += (long long)gridDim.x * kQuadGroups) {
@@ -459,7 +455,7 @@ filter_quad_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, int
 		quad_sync(bar);
 		if (ns > 1 && !(s_flag[sub][0] | s_flag[sub][1])) {
 			for (int n = 0; n < ns; n++)
-				reinterpret_cast<float2 *>(vals)[(slot0 + n) * SPC + t] = make_float2(Gn[t * nsp + n], 0.f);
+				vals[(slot0 + n) * SPC + at] = Gn[t * nsp + n];
 			if (t == 0) eq[g] = 1;
 			quad_sync(bar);
 			continue;
@@ -501,7 +497,8 @@ filter_quad_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, int
 		const float wg = s_w[sub];
 		const float wp = __fmul_rn(wg, wn[t]);
 		for (int n = 0; n < ns; n++)
-			reinterpret_cast<float2 *>(vals)[(slot0 + n) * SPC + t] = make_float2(__fmul_rn(wp, Gn[t * nsp + n]), wp);
+			vals[(slot0 + n) * SPC + at] = __fmul_rn(wp, Gn[t * nsp + n]);
+		if (t < ns) wslot[slot0 + t] = wg;
 		if (t == 0) { wgroup[g] = wg; eq[g] = 0; }
 		quad_sync(bar);
 	}
@@ -516,7 +513,7 @@ __global__ void fixup_equal_kernel(const Tile *__restrict__ tiles, int ntiles, S
                                    const float *__restrict__ win, long long g_begin, long long g_end,
                                    const uint8_t *__restrict__ nsimp, const uint8_t *__restrict__ alive,
                                    const uint8_t *__restrict__ eq, const float *__restrict__ wgroup,
-                                   float *__restrict__ vals)
+                                   float *__restrict__ vals, float *__restrict__ wslot)
 {
 	const int per = sp.C * sp.spc;
 	for (long long g = g_begin + blockIdx.x * (long long)blockDim.x + threadIdx.x; g < g_end;
@@ -529,13 +526,13 @@ __global__ void fixup_equal_kernel(const Tile *__restrict__ tiles, int ntiles, S
 			float w = 1.f;
 			for (long long q = g - 1; q >= T.g0; q--)
 				if (alive[q] && !eq[q] && nsimp[q] > n) { w = wgroup[q]; break; }
-			const int ts = term_stride(sp.C);
-			float *v = vals + (slot0 + n) * sp.spc * ts;
+			float *v = vals + (slot0 + n) * per;
 			for (int p = 0; p < sp.spc; p++) {
 				const float wp = __fmul_rn(w, win[p]);
-				for (int c = 0; c < sp.C; c++) v[p * ts + c] = __fmul_rn(wp, v[p * ts + c]);
-				v[p * ts + sp.C] = wp;
+				const int at = term_of(sp.px, p);
+				for (int c = 0; c < sp.C; c++) v[c * sp.spc + at] = __fmul_rn(wp, v[c * sp.spc + at]);
 			}
+			wslot[slot0 + n] = w;
 		}
 	}
 }
@@ -556,14 +553,14 @@ template <int STEP, int PX, int PT, int CC>
 cudaError_t launch_exact(int blocks, size_t smem, cudaStream_t st, const Image &noisy, const Image &basic,
                          const Tile *tiles, int ntiles, const StepParams &sp, const float *basis, const float *binv,
                          const float *win, long long g_begin, long long g_end, const uint8_t *nsimp,
-                         const uint32_t *idx, const uint8_t *alive, float *vals, float *wgroup,
+                         const uint32_t *idx, const uint8_t *alive, float *vals, float *wslot, float *wgroup,
                          uint8_t *eq)
 {
 	auto kern = filter_exact_kernel<STEP, PX, PT, CC>;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess) return e;
 	kern<<<blocks, kFilterThreads, smem, st>>>(noisy, basic, tiles, ntiles, sp, basis, binv, win, g_begin, g_end,
-	                                          nsimp, idx, alive, vals, wgroup, eq);
+	                                          nsimp, idx, alive, vals, wslot, wgroup, eq);
 	return cudaGetLastError();
 }
 
@@ -571,23 +568,23 @@ template <int STEP, int PX, int PT>
 cudaError_t launch_quad(int blocks, size_t smem, cudaStream_t st, const Image &noisy, const Image &basic,
                         const Tile *tiles, int ntiles, const StepParams &sp, const float *basis, const float *binv,
                         const float *win, long long g_begin, long long g_end, const uint8_t *nsimp,
-                        const uint32_t *idx, const uint8_t *alive, float *vals, float *wgroup,
+                        const uint32_t *idx, const uint8_t *alive, float *vals, float *wslot, float *wgroup,
                         uint8_t *eq)
 {
 	auto kern = filter_quad_kernel<STEP, PX, PT>;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess) return e;
 	kern<<<blocks, kQuadSub * kQuadGroups, smem, st>>>(noisy, basic, tiles, ntiles, sp, basis, binv, win, g_begin,
-	                                                  g_end, nsimp, idx, alive, vals, wgroup, eq);
+	                                                  g_end, nsimp, idx, alive, vals, wslot, wgroup, eq);
 	return cudaGetLastError();
 }
 
 #define FILTER_ARGS_NB noisy, basic, tiles, ntiles, sp, basis, binv, win, g_begin, g_end, nsimp, idx, alive, vals, \
-	    wgroup, eq
+	    wslot, wgroup, eq
 
 #define FILTER_ARGS                                                                                   \
 	blocks, smem, st, noisy, basic, tiles, ntiles, sp, basis, binv, win, g_begin, g_end, nsimp, idx, alive, \
-	    vals, wgroup, eq
+	    vals, wslot, wgroup, eq
 
 }  // namespace
 
@@ -595,7 +592,7 @@ cudaError_t launch_filter(const Image &noisy, const Image &basic, const Tile *ti
                           const StepParams &sp, const float *basis, const float *binv,
                           const float *win, long long g_begin, long long g_end,
                           const uint8_t *nsimp, const uint32_t *idx, const uint8_t *alive,
-                          float *vals, float *wgroup, uint8_t *eq, int nsm,
+                          float *vals, float *wslot, float *wgroup, uint8_t *eq, int nsm,
                           cudaStream_t st)
 {
 	if (g_end <= g_begin) return cudaSuccess;
@@ -622,7 +619,7 @@ cudaError_t launch_filter(const Image &noisy, const Image &basic, const Tile *ti
 	if (e != cudaSuccess) return e;
 	const int fb = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
 	fixup_equal_kernel<<<fb, 256, 0, st>>>(tiles, ntiles, sp, win, g_begin, g_end, nsimp, alive, eq,
-	                                       wgroup, vals);
+	                                       wgroup, vals, wslot);
 	return cudaGetLastError();
 }
 

@@ -32,7 +32,7 @@ struct Plan {
 	std::vector<int> grid;     // per tile: [xs | inverse x] [ys | inverse y] [fs | inverse t]
 	long long G = 0;
 	size_t pix = 0;            // total tile pixels (one channel)
-	size_t maxpos = 0;         // largest tile pixel count
+	long long nbins = 0;       // aggregation bins of all tiles
 };
 void determine_factor(unsigned n, unsigned &a, unsigned &b);
 // borders: null for the tiles of a run, else the six sides {x0, y0, t0, x1,
@@ -76,7 +76,7 @@ cudaError_t launch_filter(const Image &noisy, const Image &basic, const Tile *ti
                           const StepParams &sp, const float *basis, const float *binv,
                           const float *win, long long g_begin, long long g_end,
                           const uint8_t *nsimp, const uint32_t *idx, const uint8_t *alive,
-                          float *vals, float *wgroup, uint8_t *eq, int nsm,
+                          float *vals, float *wslot, float *wgroup, uint8_t *eq, int nsm,
                           cudaStream_t st);
 
 // aggregate.cu
@@ -100,24 +100,21 @@ cudaError_t launch_paste_resolve(const Tile *tiles, int ntiles, const int *grid,
                                  cudaStream_t st);
 cudaError_t launch_count_alive(const Tile *tiles, int ntiles, long long G, const uint8_t *alive,
                                unsigned *counts, cudaStream_t st);
-cudaError_t exclusive_scan(unsigned *data, size_t n, unsigned *scratch, cudaStream_t st);
-unsigned scan_kernels(size_t n);
-// launch_lists and launch_gather add the kernels they launch to *launches
-cudaError_t launch_lists(long long ga, long long gb, int np, const uint8_t *nsimp,
-                         const uint32_t *idx, const uint8_t *alive, size_t npos, unsigned *cnt,
-                         unsigned *off, unsigned *list, unsigned *scratch, unsigned *launches, cudaStream_t st);
-// Ordered gather of the slots whose origins lie in frames [t_lo, t_hi].  4x4
-// patches (quad_path): row lists (offsets in cnt) and quad lists (offsets in
-// soff), both in sl, then a merge over origin frames per quad of 4 pixels;
-// other patches: spatial lists (soff), then a merge per pixel.  cnt and soff
-// hold npos+1 entries, sl list_entries_per_member(sp) entries per slot of a
-// chunk of `members` slots.
-bool quad_path(const StepParams &sp);
-int list_entries_per_member(const StepParams &sp);
-cudaError_t launch_gather(const Tile &T, const StepParams &sp, int t_lo, int t_hi,
-                          const unsigned *off, const unsigned *list, unsigned *cnt, unsigned *soff, unsigned *sl,
-                          size_t members, unsigned *scratch, const float *vals, float *acc, float *wacc,
-                          unsigned *launches, cudaStream_t st);
+// Ordered aggregation of the groups [ga, gb): their slots listed by bin, then
+// added bin by bin in slot order.  heads holds kBinHeads + nbins words (cnt =
+// heads + kBinHeads), cursor and bins nbins words each, list
+// bin_entries_per_member(sp) words per slot of the chunk.  Adds the kernels it
+// launches to *launches.
+constexpr int kBinHeads = 4;
+struct BinArgs {
+	unsigned nbins;
+	unsigned *heads, *cnt, *cursor, *bins, *list;
+};
+int bin_entries_per_member(const StepParams &sp);
+cudaError_t launch_aggregate(const BinArgs &a, const Tile *tiles, int ntiles, const StepParams &sp, long long ga,
+                             long long gb, const uint8_t *nsimp, const uint32_t *idx, const uint8_t *alive,
+                             const float *vals, const float *wslot, const float *win, float *acc, float *wacc, int nsm,
+                             unsigned *launches, cudaStream_t st);
 cudaError_t launch_color(const Image &in, const Image &out, int forward, cudaStream_t st);
 cudaError_t launch_finalize(const Tile *tiles, int nW, int wTmp, int hTmp, const StepParams &sp,
                             const Image &noisy, const float *acc, const float *wacc,
@@ -153,7 +150,7 @@ struct LearnedArgs {
 	const float *basis, *binv, *win;
 	__nv_bfloat16 *feat;                 // features: [rows][80]
 	const float *gains;                  // apply: [rows][64], or null (no network)
-	float *vals;                         // apply: aggregation terms (estimate, weight term)
+	float *vals, *wslot;                 // apply: aggregation terms, member weights
 	float kappa;                         // apply: residual-variance fallback threshold
 	unsigned *nfallback;
 	float *sfeat, *starget;              // samples: [G][65], [G][64]

@@ -236,7 +236,8 @@ __device__ void group_body(const LearnedArgs &a, const StepParams &sp, long long
 	const float wp = wgt * win[k];
 #pragma unroll
 	for (int m = 0; m < NS; m++)
-		reinterpret_cast<float2 *>(a.vals)[(slot0 + m) * kSpc + k] = make_float2(wp * est[m], wp);
+		a.vals[(slot0 + m) * kSpc + term_of(sp.px, k)] = wp * est[m];
+	if (k < NS) a.wslot[slot0 + k] = wgt;
 }
 
 template <int MODE>
@@ -461,8 +462,9 @@ __device__ void tc_group(const LearnedArgs &a, const StepParams &sp, long long g
 		const float wp = wgt * win[p];
 #pragma unroll
 		for (int m = 0; m < NS; m++)
-			reinterpret_cast<float2 *>(a.vals)[(slot0 + m) * kSpc + p] = make_float2(wp * W.Z[p][m], wp);
+			a.vals[(slot0 + m) * kSpc + term_of(sp.px, p)] = wp * W.Z[p][m];
 	}
+	if (lane < NS) a.wslot[slot0 + lane] = wgt;
 }
 
 template <int MODE>

@@ -185,7 +185,7 @@ extern "C" bm4dof_status bm4dof_search_groups_noalloc(const float *video, const 
 	T.gf = T.gy + T.ny + T.h;
 	T.g0 = 0;
 	T.pix0 = 0;
-	T.lin0 = 0;
+	T.bin0 = 0;
 	const int sWx = (int)p->sizeSearchWindow;
 	const long long G = (long long)T.nx * T.ny * T.nf;
 	*count = (size_t)G;

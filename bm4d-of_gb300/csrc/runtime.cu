@@ -3,7 +3,7 @@
 //
 // Per step:  colour transform -> reference grid of every tile -> patch search
 // of all groups -> resolution of the mask switch-offs -> in chunks of groups:
-// group filter, origin lists, ordered gather -> normalisation, tile rebuild
+// group filter, bin lists, ordered gather -> normalisation, tile rebuild
 // and inverse colour transform.  Frames, flows, the basic estimate and the
 // aggregation buffers stay resident on the device between the two steps.
 #include <cuda_runtime.h>
@@ -66,7 +66,7 @@ struct bm4dof_ctx {
 	bool no_marks = false;       // inside a graph capture: no timing events
 	int search_ctas = 0;         // exact search CTAs per SM (0: default)
 	int search_strip = 0;        // exact search candidates per thread along a column (0: default)
-	int gather_depth = 0;        // quad gather members in flight per thread (0: 1)
+	int gather_depth = 0;        // ordered gather's staging depth (0: 1)
 	size_t held = 0;          // device bytes held in bufs
 	size_t mem_limit = 0;     // cap on held (0: none), bm4dof_set_memory_limit
 	std::recursive_mutex mu;  // calls on one context are serialised (CtxLock)
@@ -197,7 +197,8 @@ void make_plan(Plan &pl, unsigned W, unsigned H, unsigned F, unsigned nparts, co
 	pl.grid.clear();
 	pl.G = 0;
 	pl.pix = 0;
-	pl.maxpos = 0;
+	pl.nbins = 0;
+	const int bt = bin_frames(sPx, sPt);
 	for (int pp = 0; pp < pl.nH; pp++)
 		for (int q = 0; q < pl.nW; q++) {
 			Tile T;
@@ -255,11 +256,13 @@ void make_plan(Plan &pl, unsigned W, unsigned H, unsigned F, unsigned nparts, co
 			T.gf = push(fs, (int)F);
 			T.g0 = pl.G;
 			T.pix0 = (long long)pl.pix;
-			T.lin0 = pl.pix;
+			T.bin0 = pl.nbins;
+			T.nbx = (T.w + kBinX - 1) / kBinX;
+			T.nby = (T.h + kBinY - 1) / kBinY;
+			pl.nbins += (long long)T.nbx * T.nby * (((int)F + bt - 1) / bt);
 			pl.G += (long long)T.nx * T.ny * T.nf;
 			const size_t np_ = (size_t)T.w * T.h * F;
 			pl.pix += np_;
-			pl.maxpos = std::max(pl.maxpos, np_);
 			pl.tiles.push_back(T);
 		}
 }
@@ -368,8 +371,8 @@ struct StepState {
 	long long *d_blocks = nullptr;
 	unsigned long long *d_edges = nullptr;
 	float *d_acc = nullptr, *d_wacc = nullptr, *d_vals = nullptr;
-	unsigned *d_cnt = nullptr, *d_off = nullptr, *d_soff = nullptr, *d_scratch = nullptr, *d_list = nullptr,
-	         *d_sl = nullptr;
+	float *d_wslot = nullptr;
+	BinArgs bins = {0, nullptr, nullptr, nullptr, nullptr, nullptr};
 	__nv_bfloat16 *d_lfeat = nullptr;
 	float *d_lgain = nullptr, *d_gm = nullptr;
 	uint16_t *d_gw = nullptr;
@@ -561,27 +564,34 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 		SBUF("paste_counts", kPasteRounds + 3, S.paste.counts);
 	}
 
-	// shared aggregation buffers; chunks of groups whose slot terms (vals),
-	// weights, origin lists and spatial lists fit the slot budget; slot
-	// numbers must fit 26 bits
+	// shared aggregation buffers; chunks of groups whose terms, weights and
+	// bin lists take at most an eighth of the slot budget (half of a batched
+	// sequence's, which is the smaller): with 2 GiB chunks a new context
+	// allocates 14 GiB less than with whole-budget ones, and the gather still
+	// sees thousands of bins per chunk
+	if (pl.nbins > 0x7fffffffll) {
+		set_error("bm4dof: unsupported parameters: video too large");
+		return BM4DOF_ERR_UNSUPPORTED;
+	}
 	DBUF("acc", pl.pix * C, S.d_acc);
 	DBUF("wacc", pl.pix, S.d_wacc);
-	DBUF("cnt", pl.maxpos + 1, S.d_cnt);   // also the quad path's row-list offsets: ceil(w/4)*h*F + 1 entries
-	DBUF("off", pl.maxpos + 1, S.d_off);
-	DBUF("soff", pl.maxpos + 1, S.d_soff);
-	DBUF("scratch", pl.maxpos / 4096 + pl.maxpos / (4096ull * 4096ull) + 64, S.d_scratch);
-	const size_t per_group = (size_t)sp.np * ((size_t)term_stride(C) * sp.spc + 1 + (size_t)list_entries_per_member(sp)) *
+	S.bins.nbins = (unsigned)pl.nbins;
+	DBUF("bin_heads", kBinHeads + (size_t)pl.nbins, S.bins.heads);
+	DBUF("bin_cursor", (size_t)pl.nbins, S.bins.cursor);
+	DBUF("bins", (size_t)pl.nbins, S.bins.bins);
+	S.bins.cnt = S.bins.heads + kBinHeads;
+	const size_t per_group = (size_t)sp.np * ((size_t)C * sp.spc + 1 + (size_t)bin_entries_per_member(sp)) *
 	                             sizeof(float) +
 	                         (mode.learned ? (size_t)kMlpInPad * 2 + (size_t)kMlpOutN * 4 : 0);
-	size_t budget = ctx->slot_budget;
+	const size_t budget = ctx->slot_budget / (ctx->fixed_budget ? 2 : 8);
 	long long chunk = std::max<long long>(1, (long long)(budget / per_group));
-	chunk = std::min<long long>(chunk, ((1ll << 26) - 1) / sp.np);
+	chunk = std::min<long long>(chunk, (1ll << 28) / sp.np);   // list positions fit 32 bits
 	chunk = std::min<long long>(chunk, std::max<long long>(1, G));
 	S.chunk = chunk;
 	if (!mode.samples) {
-		DBUF("vals", (size_t)chunk * sp.np * term_stride(C) * sp.spc, S.d_vals);
-		DBUF("list", (size_t)chunk * sp.np, S.d_list);
-		DBUF("slist", (size_t)chunk * sp.np * list_entries_per_member(sp), S.d_sl);
+		DBUF("vals", (size_t)chunk * sp.np * C * sp.spc, S.d_vals);
+		DBUF("wslot", (size_t)chunk * sp.np, S.d_wslot);
+		DBUF("bin_list", (size_t)chunk * sp.np * bin_entries_per_member(sp), S.bins.list);
 	}
 	if (mode.learned) {
 		DBUF("lfeat", (size_t)chunk * kMlpInPad, S.d_lfeat);
@@ -704,53 +714,39 @@ bm4dof_status launch_step(bm4dof_ctx *ctx, int slot, const Image &noisy, const I
 	// ---- filter + ordered aggregation, in chunks of groups --------------------
 	CK(cudaMemsetAsync(S.d_acc, 0, sizeof(float) * pl.pix * C, st));
 	CK(cudaMemsetAsync(S.d_wacc, 0, sizeof(float) * pl.pix, st));
+	// (a chunk may span tiles: every tile has its own pixels and bins)
 	const long long chunk = S.chunk;
-	for (int ti = 0; ti < ntiles; ti++) {
-		const Tile &T = pl.tiles[ti];
-		const long long gend = T.g0 + (long long)T.nx * T.ny * T.nf;
-		const size_t npos = (size_t)T.w * T.h * F;
-		for (long long ga = T.g0; ga < gend; ga += chunk) {
-			const long long gb = std::min(gend, ga + chunk);
-			{
-				Mark m(ctx, T_FILTER);
-				if (mode.learned) {
-					la.ga = ga;
-					la.gb = gb;
-					la.feat = S.d_lfeat;
-					la.vals = S.d_vals;
-					la.gains = nullptr;
-					if (ctx->has_gain) {
-						CK(launch_learned(kLearnedFeatures, la, sp, ctx->nsm, st));
-						CK(launch_mlp_forward(reinterpret_cast<const uint16_t *>(S.d_lfeat), gb - ga,
-						                      mlp_weights(S.d_gw, S.d_gm), S.d_lgain, ctx->nsm, st));
-						ctx->launches += 2;
-						la.gains = S.d_lgain;
-					}
-					CK(launch_learned(kLearnedApply, la, sp, ctx->nsm, st));
-					ctx->launches++;
-				} else {
-					CK(launch_filter(noisy, basic, S.d_tiles, ntiles, sp, S.d_basis, S.d_binv, S.d_win, ga, gb,
-					                 S.d_nsimp, S.d_idx, S.d_alive, S.d_vals, S.d_wgroup, S.d_eq,
-					                 ctx->nsm, st));
+	for (long long ga = 0; ga < G; ga += chunk) {
+		const long long gb = std::min(G, ga + chunk);
+		{
+			Mark m(ctx, T_FILTER);
+			if (mode.learned) {
+				la.ga = ga;
+				la.gb = gb;
+				la.feat = S.d_lfeat;
+				la.vals = S.d_vals;
+				la.wslot = S.d_wslot;
+				la.gains = nullptr;
+				if (ctx->has_gain) {
+					CK(launch_learned(kLearnedFeatures, la, sp, ctx->nsm, st));
+					CK(launch_mlp_forward(reinterpret_cast<const uint16_t *>(S.d_lfeat), gb - ga,
+					                      mlp_weights(S.d_gw, S.d_gm), S.d_lgain, ctx->nsm, st));
 					ctx->launches += 2;
+					la.gains = S.d_lgain;
 				}
+				CK(launch_learned(kLearnedApply, la, sp, ctx->nsm, st));
+				ctx->launches++;
+			} else {
+				CK(launch_filter(noisy, basic, S.d_tiles, ntiles, sp, S.d_basis, S.d_binv, S.d_win, ga, gb,
+				                 S.d_nsimp, S.d_idx, S.d_alive, S.d_vals, S.d_wslot, S.d_wgroup, S.d_eq,
+				                 ctx->nsm, st));
+				ctx->launches += 2;
 			}
-			{
-				Mark m(ctx, T_AGG);
-				CK(launch_lists(ga, gb, sp.np, S.d_nsimp, S.d_idx, S.d_alive, npos, S.d_cnt, S.d_off, S.d_list,
-				                S.d_scratch, &ctx->launches, st));
-				// origin frames of the chunk's member patches: the temporal search
-				// range of a reference frame t lies within t -/+ (wtb + wtf)
-				const long long fa = (ga - T.g0) / ((long long)T.nx * T.ny);
-				const long long fb = (gb - 1 - T.g0) / ((long long)T.nx * T.ny);
-				const int ta = pl.grid[T.gf + (int)fa], tb = pl.grid[T.gf + (int)fb];
-				const int reach = sp.wtb + sp.wtf;
-				const int t_lo = std::max(0, ta - reach);
-				const int t_hi = std::min((int)F - sp.pt, tb + reach);
-				CK(launch_gather(T, sp, t_lo, t_hi, S.d_off, S.d_list, S.d_cnt, S.d_soff, S.d_sl,
-				                 (size_t)chunk * sp.np, S.d_scratch, S.d_vals, S.d_acc + T.pix0 * C,
-				                 S.d_wacc + T.pix0, &ctx->launches, st));
-			}
+		}
+		{
+			Mark m(ctx, T_AGG);
+			CK(launch_aggregate(S.bins, S.d_tiles, ntiles, sp, ga, gb, S.d_nsimp, S.d_idx, S.d_alive, S.d_vals,
+			                    S.d_wslot, S.d_win, S.d_acc, S.d_wacc, ctx->nsm, &ctx->launches, st));
 		}
 	}
 

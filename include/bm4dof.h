@@ -293,8 +293,9 @@ typedef struct bm4dof_tuning {
 	                          column: 7 or 21; 0: 21 for windows of 15 rows or
 	                          more (4x4x4 patches at 6 CTAs per SM; at 4 CTAs
 	                          per SM and for other patches the strip is 7)      */
-	unsigned gather_depth; /* members in flight per thread of the ordered
-	                          gather (4x4 patches): 1 or 2; 0: 1                */
+	unsigned gather_depth; /* staging depth of the ordered gather (grey 4x4
+	                          patches): 1 (4 members in flight per thread) or
+	                          2 (8); 0: 1                                       */
 } bm4dof_tuning;
 
 /* Denoises n sequences (flags: BM4DOF_MIXED_PRECISION, BM4DOF_LEARNED,
