@@ -28,7 +28,7 @@ PSNR_CLI = os.path.join(OUT, "psnr")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC",
            "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
-SOURCES = ["search.cu", "search_vbm3d.cu", "search_tc.cu", "filter.cu", "aggregate.cu", "runtime.cu", "noalloc.cu",
+SOURCES = ["search.cu", "search_block.cu", "search_vbm3d.cu", "search_tc.cu", "filter.cu", "aggregate.cu", "runtime.cu", "noalloc.cu",
            "mlp.cu", "learned.cu", "tvl1.cu", "peaks.cu",
            "params.cpp", "basis.cpp"]
 

@@ -38,6 +38,8 @@ struct Tile {                     // one spatial tile (crop) of one step
 	long long pix0;               // first pixel of this tile's aggregation buffers
 	long long bin0;               // first aggregation bin of this tile
 	int nbx, nby;                 // its bins along x and y
+	long long blk0;               // first 2 x 2 block of reference patches (search_block.cu)
+	int bkx, bky, prx, pry;       // blocks along x and y, and how many of them are regular pairs
 	int bx0, by0, bx1, by1;       // crop touches an inner border (nldct.cpp:520-525)
 };
 
@@ -51,8 +53,8 @@ struct StepParams {               // resolved parameters of one step
 	float sigma, beta, tau2;      // tau2 = tau*tau*px*px*pt (nldct.cpp:1158)
 	int use_flow;
 	float beta1;                  // learned form: hard threshold of the non-mean Haar rows
-	int search_ctas;              // exact search: CTAs per SM (4 or 6; 0 = default)
-	int search_strip;             // exact search: candidates per thread along a column (7 or 21; 0 = default)
+	int search_ctas;              // per-group search: CTAs per SM (4 or 6; 0 = default)
+	int search_strip;             // 7: per-group search with strips of 7 candidates; 21, 0: default
 	int gather_depth;             // ordered gather: staging depth (1 or 2; 0 = 1)
 	float beta_mean;              // betaMean (order-invariant filtering)
 	int order_inv;                // orderInvariance

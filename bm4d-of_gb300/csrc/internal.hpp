@@ -33,6 +33,9 @@ struct Plan {
 	long long G = 0;
 	size_t pix = 0;            // total tile pixels (one channel)
 	long long nbins = 0;       // aggregation bins of all tiles
+	int step = 0;              // offSet, the reference grid's step in x and y
+	long long nblocks = 0;     // 2 x 2 blocks of reference patches of all tiles
+	bool blocks_ok = true;     // every group lies in a block
 };
 void determine_factor(unsigned n, unsigned &a, unsigned &b);
 // borders: null for the tiles of a run, else the six sides {x0, y0, t0, x1,
@@ -45,11 +48,24 @@ int search_frames_max(const StepParams &sp);
 cudaError_t launch_traj(const Image &ffl, const Image &bfl, const Tile *tiles, int ntiles, const int *grid,
                         const StepParams &sp, long long G, uint32_t *traj, cudaStream_t st);
 // With glist, the groups glist[0 .. *gcount) (a device-side count, at most
-// g_end - g_begin of them) instead of the range [g_begin, g_end).
+// g_end - g_begin of them) instead of the range [g_begin, g_end), unless the
+// device-side flag *all is set.
 cudaError_t launch_search(const Image &src, const Tile *tiles, int ntiles, const int *grid,
                           const uint32_t *traj, const StepParams &sp, long long g_begin, long long g_end,
                           uint8_t *nsimp, uint32_t *idx, int *err, int nsm, cudaStream_t st,
-                          const uint32_t *glist = nullptr, const unsigned *gcount = nullptr);
+                          const uint32_t *glist = nullptr, const unsigned *gcount = nullptr,
+                          const unsigned *all = nullptr);
+
+// search_block.cu: the exact search by 2 x 2 blocks of reference patches.  The
+// groups it leaves to launch_search are listed in glist / *gcount; when the
+// source holds values it cannot take (*bad_source set) it does nothing.  Both
+// words must be zero before.  src needs block_search_guard floats of memory
+// before and after it (their values do not matter).
+bool block_search_supported(const StepParams &sp, const Plan &pl);
+size_t block_search_guard(int pitch);
+cudaError_t launch_search_block(const Image &src, const Tile *tiles, int ntiles, const int *grid, const uint32_t *traj,
+                                const StepParams &sp, int step, long long nblocks, uint8_t *nsimp, uint32_t *idx,
+                                uint32_t *glist, unsigned *gcount, unsigned *bad_source, int nsm, cudaStream_t st);
 
 // search_vbm3d.cu (the reference's VBM3D_SEARCH build)
 bool vbm3d_check(const StepParams &sp, const std::vector<Tile> &tiles, std::string &why);

@@ -64,8 +64,8 @@ struct bm4dof_ctx {
 	size_t slot_budget = 0;   // bytes of per-chunk aggregation terms
 	bool fixed_budget = false;   // batched children: slot_budget set by the tuning
 	bool no_marks = false;       // inside a graph capture: no timing events
-	int search_ctas = 0;         // exact search CTAs per SM (0: default)
-	int search_strip = 0;        // exact search candidates per thread along a column (0: default)
+	int search_ctas = 0;         // per-group search: CTAs per SM (0: default)
+	int search_strip = 0;        // 7: per-group search (0, 21: default)
 	int gather_depth = 0;        // ordered gather's staging depth (0: 1)
 	size_t held = 0;          // device bytes held in bufs
 	size_t mem_limit = 0;     // cap on held (0: none), bm4dof_set_memory_limit
@@ -126,6 +126,15 @@ bm4dof_status dbuf(bm4dof_ctx *ctx, const char *name, size_t count, T **out)
 	*out = static_cast<T *>(b.p);
 	return BM4DOF_OK;
 }
+
+// A full-frame video the patch search reads: with room on both sides for the
+// pixels that a block of reference patches reaches past it.
+#define VBUF(name, count, pitch, ptr)                                      \
+	do {                                                                   \
+		const size_t guard_ = block_search_guard((int)(pitch));            \
+		DBUF(name, (count) + 2 * guard_, ptr);                             \
+		ptr += guard_;                                                     \
+	} while (0)
 
 #define DBUF(name, count, ptr)                                 \
 	do {                                                       \
@@ -198,6 +207,9 @@ void make_plan(Plan &pl, unsigned W, unsigned H, unsigned F, unsigned nparts, co
 	pl.G = 0;
 	pl.pix = 0;
 	pl.nbins = 0;
+	pl.nblocks = 0;
+	pl.blocks_ok = true;
+	pl.step = (int)p.offSet;
 	const int bt = bin_frames(sPx, sPt);
 	for (int pp = 0; pp < pl.nH; pp++)
 		for (int q = 0; q < pl.nW; q++) {
@@ -260,6 +272,20 @@ void make_plan(Plan &pl, unsigned W, unsigned H, unsigned F, unsigned nparts, co
 			T.nbx = (T.w + kBinX - 1) / kBinX;
 			T.nby = (T.h + kBinY - 1) / kBinY;
 			pl.nbins += (long long)T.nbx * T.nby * (((int)F + bt - 1) / bt);
+			// 2 x 2 blocks of reference patches: the regular columns in pairs, then
+			// each left-over one beside a missing left neighbour, offSet away
+			auto pairs = [&pl, &p](const std::vector<int> &v) {
+				size_t n = v.size();
+				if (n > 1 && v[n - 1] - v[n - 2] != (int)p.offSet) n--;
+				if (2 * (n / 2) < v.size() && v[2 * (n / 2)] < (int)p.offSet) pl.blocks_ok = false;
+				return (int)(n / 2);
+			};
+			T.prx = pairs(xs);
+			T.pry = pairs(ys);
+			T.bkx = T.nx - T.prx;
+			T.bky = T.ny - T.pry;
+			T.blk0 = pl.nblocks;
+			pl.nblocks += (long long)T.bkx * T.bky * T.nf;
 			pl.G += (long long)T.nx * T.ny * T.nf;
 			const size_t np_ = (size_t)T.w * T.h * F;
 			pl.pix += np_;
@@ -356,6 +382,7 @@ struct StepState {
 	StepParams sp;
 	long long G = 0, chunk = 0;
 	bool tc_search = false;      // tcgen05 pre-screen + certified re-rank (search_tc.cu)
+	bool block_search = false;   // exact search by 2 x 2 blocks (search_block.cu)
 	size_t nblocks = 0;
 	PasteScratch paste = {nullptr, nullptr, nullptr, nullptr, nullptr};   // doPasteBoost only
 	Tile *d_tiles = nullptr;
@@ -363,10 +390,11 @@ struct StepState {
 	float *d_basis = nullptr, *d_binv = nullptr, *d_win = nullptr;
 	uint8_t *d_nsimp = nullptr, *d_alive = nullptr, *d_eq = nullptr, *d_killed = nullptr;
 	uint32_t *d_idx = nullptr, *d_traj = nullptr;
-	uint32_t *d_cand = nullptr, *d_fb = nullptr;   // tc_search: candidates, exact-search list
+	uint32_t *d_cand = nullptr, *d_fb = nullptr;   // tc_search: candidates; groups for the per-group search
 	float *d_lb = nullptr, *d_thr0 = nullptr;       // tc_search: bound on the dropped candidates, anchors
 	float *d_wgroup = nullptr;
-	unsigned *d_small = nullptr;          // [0] edges, [3] fallbacks, [4] exact-search list, [5] tc status,
+	unsigned *d_small = nullptr;          // [0] edges, [1] groups left by the block search, [2] its source
+	                                      // is not finite, [3] fallbacks, [4] exact-search list, [5] tc status,
 	                                      // [6] uncertified re-ranks, [64..] per-tile counts
 	long long *d_blocks = nullptr;
 	unsigned long long *d_edges = nullptr;
@@ -507,6 +535,7 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 	}
 	std::vector<float> win = make_window(p.agg_window != 0, sp.px, sp.pt);
 	S.tc_search = mode.mixed && tc_supported(sp, pl.tiles);
+	S.block_search = !sp.vbm3d && !S.tc_search && block_search_supported(sp, pl);
 	std::vector<long long> blocks;
 	if (S.tc_search) tc_blocks(pl.tiles, blocks);
 	S.nblocks = blocks.size();
@@ -554,8 +583,8 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 		SBUF("tc_cand", (size_t)G * 32, S.d_cand);
 		SBUF("tc_lb", G, S.d_lb);
 		SBUF("tc_thr0", G, S.d_thr0);
-		SBUF("tc_exact", G, S.d_fb);
 	}
+	if (S.tc_search || S.block_search) SBUF("search_list", G, S.d_fb);
 	if (sp.paste) {
 		SBUF("paste_pending", G, S.paste.pending);
 		SBUF("paste_state", G, S.paste.state);
@@ -655,6 +684,14 @@ bm4dof_status launch_step(bm4dof_ctx *ctx, int slot, const Image &noisy, const I
 			CK(launch_search(src, S.d_tiles, ntiles, S.d_grid, S.d_traj, sp, 0, G, S.d_nsimp, S.d_idx, nullptr,
 			                 ctx->nsm, st, S.d_fb, S.d_small + 4));
 			ctx->launches += 5;
+		} else if (S.block_search) {
+			const Image &src = on_noisy ? noisy : basic;
+			CK(launch_traj(ffl, bfl, S.d_tiles, ntiles, S.d_grid, sp, G, S.d_traj, st));
+			CK(launch_search_block(src, S.d_tiles, ntiles, S.d_grid, S.d_traj, sp, pl.step, pl.nblocks, S.d_nsimp, S.d_idx,
+			                       S.d_fb, S.d_small + 1, S.d_small + 2, ctx->nsm, st));
+			CK(launch_search(src, S.d_tiles, ntiles, S.d_grid, S.d_traj, sp, 0, G, S.d_nsimp, S.d_idx, nullptr,
+			                 ctx->nsm, st, S.d_fb, S.d_small + 1, S.d_small + 2));
+			ctx->launches += 4;
 		} else {
 			CK(launch_traj(ffl, bfl, S.d_tiles, ntiles, S.d_grid, sp, G, S.d_traj, st));
 			CK(launch_search(on_noisy ? noisy : basic, S.d_tiles, ntiles, S.d_grid, S.d_traj, sp, 0, G, S.d_nsimp,
@@ -1014,15 +1051,15 @@ bm4dof_status prepare_run(bm4dof_ctx *ctx, RunArgs &r)
 	m2.learned = r.learned;
 	for (int pass = 0; pass < 2; pass++) {
 		// the second pass allocates nothing: every address is final after it
-		DBUF("noisy", nv, r.d_noisy);
-		DBUF("basic_rgb", nv, r.d_basic);
+		VBUF("noisy", nv, P, r.d_noisy);
+		VBUF("basic_rgb", nv, P, r.d_basic);
 		DBUF("final", nv, r.d_final);
 		if (r.use_flow) {
 			DBUF("fflow", P * r.H * 2 * r.F, r.d_ff);
 			DBUF("bflow", P * r.H * 2 * r.F, r.d_bf);
 		}
-		if ((r.run1 && r.yuv1) || (r.run2 && r.yuv2)) DBUF("noisy_yuv", nv, r.d_noisy_yuv);
-		if (r.run2 && r.yuv2 && !r.learned) DBUF("basic_yuv", nv, r.d_basic_yuv);
+		if ((r.run1 && r.yuv1) || (r.run2 && r.yuv2)) VBUF("noisy_yuv", nv, P, r.d_noisy_yuv);
+		if (r.run2 && r.yuv2 && !r.learned) VBUF("basic_yuv", nv, P, r.d_basic_yuv);
 		bm4dof_status e;
 		if (r.run1 && (e = prepare_step(ctx, 0, 1, r.p1, r.W, r.H, r.C, r.F, r.use_flow, r.nparts, r.mode)) != BM4DOF_OK)
 			return e;
@@ -1540,8 +1577,8 @@ bm4dof_status bm4dof_autotune(bm4dof_ctx *ctx, bm4dof_sequence *seqs, unsigned n
 		if (ms < best_ms) { best_ms = ms; cur = t; }
 	}
 	{
-		// the exact search's tile shape: 21 or 7 candidates per thread along a
-		// window column at 6 CTAs per SM, or strips of 7 at 4 CTAs per SM
+		// the exact search's tile shape: by blocks of patches, or per group with
+		// strips of 7 candidates at 6 or 4 CTAs per SM
 		const bm4dof_tuning b2 = cur;
 		const unsigned shapes[2][2] = {{6, 7}, {4, 7}};
 		for (const auto &sh : shapes) {
@@ -1687,8 +1724,8 @@ bm4dof_status bm4dof_gain_samples(bm4dof_ctx *ctx, const float *noisy, const flo
 	ctx->launches = 0;
 	const size_t P = (W + 7) / 8 * 8, nv = P * H * F;
 	float *d_noisy, *d_basic, *d_ff = nullptr, *d_bf = nullptr;
-	DBUF("noisy", nv, d_noisy);
-	DBUF("basic_rgb", nv, d_basic);
+	VBUF("noisy", nv, P, d_noisy);
+	VBUF("basic_rgb", nv, P, d_basic);
 	Image in = image(d_noisy, W, H, 1, F), bas = image(d_basic, W, H, 1, F);
 	Image ff = image(nullptr, W, H, 2, F), bf = image(nullptr, W, H, 2, F);
 	bm4dof_status s;
@@ -1706,8 +1743,8 @@ bm4dof_status bm4dof_gain_samples(bm4dof_ctx *ctx, const float *noisy, const flo
 		return BM4DOF_ERR_ARGUMENT;
 	}
 	// addresses of the inputs after the step's allocations
-	DBUF("noisy", nv, d_noisy);
-	DBUF("basic_rgb", nv, d_basic);
+	VBUF("noisy", nv, P, d_noisy);
+	VBUF("basic_rgb", nv, P, d_basic);
 	in.p = d_noisy;
 	bas.p = d_basic;
 	if (fflow) {

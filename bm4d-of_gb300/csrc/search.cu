@@ -89,6 +89,7 @@ struct SearchArgs {
 	long long g_begin, g_end;
 	const uint32_t *glist;   // when set: the groups glist[0 .. *gcount) instead of [g_begin, g_end)
 	const unsigned *gcount;
+	const unsigned *all;     // with glist: when *all is set, the whole range after all
 	uint8_t *nsimp;
 	uint32_t *idx;
 };
@@ -292,9 +293,10 @@ search_kernel(Image src, StepParams sp, SearchArgs a)
 
 	const int tid = threadIdx.x;
 	const int chn = sp.chn_search;
-	const long long ng = a.glist ? (long long)*a.gcount : a.g_end - a.g_begin;
+	const bool listed = a.glist && !(a.all && *a.all);
+	const long long ng = listed ? (long long)*a.gcount : a.g_end - a.g_begin;
 	for (long long gi = blockIdx.x; gi < ng; gi += gridDim.x) {
-		const long long g = a.glist ? (long long)a.glist[gi] : a.g_begin + gi;
+		const long long g = listed ? (long long)a.glist[gi] : a.g_begin + gi;
 		if (tid < 32) plan_group(a, sp, g, R, fw, s_nframes, s_ncand, s_nitems, s_tile, s_x, s_y, s_t);
 		__syncthreads();
 		const Tile T = a.tiles[s_tile];
@@ -403,7 +405,7 @@ cudaError_t launch_traj(const Image &ffl, const Image &bfl, const Tile *tiles, i
 cudaError_t launch_search(const Image &src, const Tile *tiles, int ntiles, const int *grid,
                           const uint32_t *traj, const StepParams &sp, long long g_begin, long long g_end,
                           uint8_t *nsimp, uint32_t *idx, int *err, int nsm, cudaStream_t st, const uint32_t *glist,
-                          const unsigned *gcount)
+                          const unsigned *gcount, const unsigned *all)
 {
 	if (g_end <= g_begin) return cudaSuccess;
 	if (sp.np <= 1 && !glist) {
@@ -422,6 +424,7 @@ cudaError_t launch_search(const Image &src, const Tile *tiles, int ntiles, const
 	a.g_end = g_end;
 	a.glist = glist;
 	a.gcount = gcount;
+	a.all = all;
 	a.nsimp = nsimp;
 	a.idx = idx;
 	(void)err;

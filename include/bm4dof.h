@@ -288,11 +288,13 @@ typedef struct bm4dof_tuning {
 	unsigned branches;     /* concurrent streams in the graph; 0: min(n, 16)     */
 	unsigned slot_mb;      /* per sequence: MB of aggregation terms per chunk
 	                          (the depth of group staging); 0: 1024              */
-	unsigned search_ctas;  /* exact search CTAs per SM: 4 or 6; 0: 6             */
-	unsigned search_strip; /* exact search candidates per thread along a window
-	                          column: 7 or 21; 0: 21 for windows of 15 rows or
-	                          more (4x4x4 patches at 6 CTAs per SM; at 4 CTAs
-	                          per SM and for other patches the strip is 7)      */
+	unsigned search_ctas;  /* per-group exact search, CTAs per SM: 4 or 6; 0: 6  */
+	unsigned search_strip; /* 21 or 0: the exact search by blocks of 2 x 2
+	                          neighbouring patches where the patch shape and grid
+	                          allow it (else per group: 21 candidates per thread
+	                          along a window column, 7 for windows under 15 rows);
+	                          7: per group, 7 candidates per thread (so does
+	                          search_ctas 4)                                    */
 	unsigned gather_depth; /* staging depth of the ordered gather (grey 4x4
 	                          patches): 1 (4 members in flight per thread) or
 	                          2 (8); 0: 1                                       */
