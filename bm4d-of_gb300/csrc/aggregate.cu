@@ -390,7 +390,7 @@ __global__ void bin_alloc_kernel(unsigned nbins, const unsigned *__restrict__ cn
 	}
 }
 
-// Adds a 4-row column of terms to the rows R .. R + 3 of a lane's 8 sums.  The
+// Adds a 4-row column of terms w * v to the rows R .. R + 3 of a lane's 8 sums.  The
 // markers keep the compiler from merging the cases of R into one that indexes
 // the sums dynamically, which would put them in local memory.
 template <int R, int CC>
@@ -403,7 +403,7 @@ __device__ __forceinline__ void add_rows(float (&a)[8][CC], float (&wa)[8], cons
 #pragma unroll
 			for (int c = 0; c < CC; c++) {
 				const float t = h == 0 ? v[c].x : h == 1 ? v[c].y : h == 2 ? v[c].z : v[c].w;
-				a[(R + h) & 7][c] = __fadd_rn(a[(R + h) & 7][c], t);
+				a[(R + h) & 7][c] = __fadd_rn(a[(R + h) & 7][c], __fmul_rn(w, t));
 			}
 			wa[(R + h) & 7] = __fadd_rn(wa[(R + h) & 7], w);
 		}
@@ -666,7 +666,7 @@ bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, lon
 									for (int s = 0; s < NS; s++)
 										if ((fm[u] >> (s >> 1) & 1u) && ok[u][s & 1]) {
 #pragma unroll
-											for (int c = 0; c < CC; c++) a[s][c] = __fadd_rn(a[s][c], v[u][s][c]);
+											for (int c = 0; c < CC; c++) a[s][c] = __fadd_rn(a[s][c], __fmul_rn(wt[u][s & 1], v[u][s][c]));
 											wa[s] = __fadd_rn(wa[s], wt[u][s & 1]);
 										}
 							}

@@ -119,6 +119,32 @@ bool make_basis(int transform, unsigned px, unsigned pt, std::vector<float> &bas
 	return true;
 }
 
+bool dct4_magnitudes(const std::vector<float> &basis, const std::vector<float> &binv, float mag[3])
+{
+	if (basis.size() != 64 * 64 || binv != basis) return false;
+	const std::vector<float> a = dct_1d(4);
+	const float m[3] = {a[0], a[4], a[5]};   // even k; k = 1 at the outer and inner pixels
+	float s[4][4];
+	for (int k = 0; k < 4; k++)
+		for (int n = 0; n < 4; n++) {
+			const bool outer = n == 0 || n == 3;
+			s[k][n] = (k & 1) == 0 ? m[0] : ((k == 1) == outer ? m[1] : m[2]);
+			if (a[k * 4 + n] < 0.f) s[k][n] = -s[k][n];
+			const bool neg = k == 1 ? n >= 2 : k == 2 ? (n == 1 || n == 2) : k == 3 ? (n & 1) != 0 : false;
+			if ((s[k][n] < 0.f) != neg) return false;
+		}
+	size_t i = 0;
+	for (int kt = 0; kt < 4; kt++)
+		for (int ky = 0; ky < 4; ky++)
+			for (int kx = 0; kx < 4; kx++)
+				for (int nt = 0; nt < 4; nt++)
+					for (int ny = 0; ny < 4; ny++)
+						for (int nx = 0; nx < 4; nx++, i++)
+							if (basis[i] != s[kx][nx] * s[ky][ny] * s[kt][nt]) return false;
+	for (int j = 0; j < 3; j++) mag[j] = m[j];
+	return true;
+}
+
 std::vector<float> make_window(bool agg, unsigned px, unsigned pt)
 {
 	std::vector<float> w((size_t)px * px * pt, 1.f);

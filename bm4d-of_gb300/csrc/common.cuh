@@ -62,12 +62,13 @@ struct StepParams {               // resolved parameters of one step
 	int wxp, npf;                 // sizeSearchWindowPred, nSimilarPatchesPred
 	float dsub_bias;              // dsub*dsub*255 (nldct.cpp:921)
 	int paste;                    // doPasteBoost
+	float dct4[3];                // 4x4x4 DCT: the basis' magnitudes per axis (filter.cu); 0: another basis
 };
 
 // Aggregation terms of a chunk of groups: for slot s (one member of one
-// group), channel c and patch element p, the weighted estimate
-// (w * window[p]) * ghat at vals[(s * C + c) * spc + term_of(px, p)], and the
-// member's weight w at wslot[s] (the gather forms w * window[p] itself).  4x4
+// group), channel c and patch element p, the estimate ghat at
+// vals[(s * C + c) * spc + term_of(px, p)], and the member's weight w at
+// wslot[s] (the gather forms (w * window[p]) * ghat itself).  4x4
 // patches hold each frame's elements column by column, so that the gather's
 // lanes read the four rows of a column with one load.
 __host__ __device__ __forceinline__ int term_of(int px, int p)

@@ -21,6 +21,9 @@ void clear_error();
 // mat.patch_basis / mat.patch_basis_inv (src/core/nldct.cpp:572-696).
 bool make_basis(int transform, unsigned px, unsigned pt, std::vector<float> &basis,
                 std::vector<float> &binv);
+// Whether a 4x4x4 basis is the separable DCT with three magnitudes per axis that
+// the warp filter computes it as; mag receives them.
+bool dct4_magnitudes(const std::vector<float> &basis, const std::vector<float> &binv, float mag[3]);
 // Aggregation window (src/core/nldct.cpp:698-737).
 std::vector<float> make_window(bool agg, unsigned px, unsigned pt);
 
@@ -90,7 +93,7 @@ cudaError_t tc_selftest(const uint16_t *A, const uint16_t *B, float *D, int *sta
 size_t filter_smem_bytes(const StepParams &sp);
 cudaError_t launch_filter(const Image &noisy, const Image &basic, const Tile *tiles, int ntiles,
                           const StepParams &sp, const float *basis, const float *binv,
-                          const float *win, long long g_begin, long long g_end,
+                          long long g_begin, long long g_end,
                           const uint8_t *nsimp, const uint32_t *idx, const uint8_t *alive,
                           float *vals, float *wslot, float *wgroup, uint8_t *eq, int nsm,
                           cudaStream_t st);

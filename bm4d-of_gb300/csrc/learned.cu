@@ -233,10 +233,9 @@ __device__ void group_body(const LearnedArgs &a, const StepParams &sp, long long
 	}
 	const float wgt = 1.f / (sigma2 * fmaxf(w2sum, 1e-3f));
 	const long long slot0 = r * sp.np;
-	const float wp = wgt * win[k];
 #pragma unroll
 	for (int m = 0; m < NS; m++)
-		a.vals[(slot0 + m) * kSpc + term_of(sp.px, k)] = wp * est[m];
+		a.vals[(slot0 + m) * kSpc + term_of(sp.px, k)] = est[m];
 	if (k < NS) a.wslot[slot0 + k] = wgt;
 }
 
@@ -459,10 +458,9 @@ __device__ void tc_group(const LearnedArgs &a, const StepParams &sp, long long g
 #pragma unroll
 	for (int h = 0; h < 2; h++) {
 		const int p = lane + 32 * h;
-		const float wp = wgt * win[p];
 #pragma unroll
 		for (int m = 0; m < NS; m++)
-			a.vals[(slot0 + m) * kSpc + term_of(sp.px, p)] = wp * W.Z[p][m];
+			a.vals[(slot0 + m) * kSpc + term_of(sp.px, p)] = W.Z[p][m];
 	}
 	if (lane < NS) a.wslot[slot0 + lane] = wgt;
 }

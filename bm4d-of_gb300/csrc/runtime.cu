@@ -533,6 +533,7 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 		set_error("VideoNLB::processNlBayes: bior1_5 transform is only implemented for patches of size 8 x 8 x pt.");
 		return BM4DOF_ERR_BIOR_SIZE;
 	}
+	if (!(sp.px == 4 && sp.pt == 4 && dct4_magnitudes(basis, binv, sp.dct4))) sp.dct4[0] = sp.dct4[1] = sp.dct4[2] = 0.f;
 	std::vector<float> win = make_window(p.agg_window != 0, sp.px, sp.pt);
 	S.tc_search = mode.mixed && tc_supported(sp, pl.tiles);
 	S.block_search = !sp.vbm3d && !S.tc_search && block_search_supported(sp, pl);
@@ -774,7 +775,7 @@ bm4dof_status launch_step(bm4dof_ctx *ctx, int slot, const Image &noisy, const I
 				CK(launch_learned(kLearnedApply, la, sp, ctx->nsm, st));
 				ctx->launches++;
 			} else {
-				CK(launch_filter(noisy, basic, S.d_tiles, ntiles, sp, S.d_basis, S.d_binv, S.d_win, ga, gb,
+				CK(launch_filter(noisy, basic, S.d_tiles, ntiles, sp, S.d_basis, S.d_binv, ga, gb,
 				                 S.d_nsimp, S.d_idx, S.d_alive, S.d_vals, S.d_wslot, S.d_wgroup, S.d_eq,
 				                 ctx->nsm, st));
 				ctx->launches += 2;
