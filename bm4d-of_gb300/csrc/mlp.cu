@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -62,13 +63,12 @@ __device__ __forceinline__ uint32_t ld_u32(const bf16 *p) { return *reinterpret_
 
 // One dense layer for the 16 rows [wr, wr+16) of a warp: out = act(in . W + b)
 // with in a bf16 shared tile of K columns and Wt[N][K] in global memory.
-// ACT 0: GELU into the bf16 shared tile `out` (and, when training, the
-// pre-activations to P and the activations to H in global memory);
-// ACT 1: sigmoid into the float rows of `gout`.
-template <int K, int N, int ACT, bool TRAIN>
+// ACT 0: GELU into the bf16 shared tile `out`; ACT 1: sigmoid into the float rows
+// of `gout`.
+template <int K, int N, int ACT>
 __device__ __forceinline__ void dense(const bf16 *in, bf16 *out, const bf16 *__restrict__ Wt,
                                       const float *__restrict__ bias, int wr, long long row0, long long n,
-                                      float *gout, float *P, bf16 *H)
+                                      float *gout)
 {
 	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll 1
@@ -103,12 +103,6 @@ __device__ __forceinline__ void dense(const bf16 *in, bf16 *out, const bf16 *__r
 					const bf16 o0 = __float2bfloat16_rn(gelu(v0)), o1 = __float2bfloat16_rn(gelu(v1));
 					out[r * kActStride + c] = o0;
 					out[r * kActStride + c + 1] = o1;
-					if (TRAIN && row < n) {
-						P[row * N + c] = v0;
-						P[row * N + c + 1] = v1;
-						H[row * N + c] = o0;
-						H[row * N + c + 1] = o1;
-					}
 				} else if (row < n) {
 					gout[row * N + c] = 1.f / (1.f + expf(-v0));
 					gout[row * N + c + 1] = 1.f / (1.f + expf(-v1));
@@ -120,10 +114,8 @@ __device__ __forceinline__ void dense(const bf16 *in, bf16 *out, const bf16 *__r
 
 // Forward pass over n feature rows.  Each warp owns 16 rows of the CTA's two
 // activation tiles, so the layers need only warp-level synchronisation.
-template <bool TRAIN>
 __global__ void __launch_bounds__(128)
-mlp_forward_kernel(const bf16 *__restrict__ X, long long n, MlpWeights w, float *__restrict__ out,
-                   float *P1, bf16 *H1, float *P2, bf16 *H2)
+mlp_forward_kernel(const bf16 *__restrict__ X, long long n, MlpWeights w, float *__restrict__ out)
 {
 	extern __shared__ __align__(16) unsigned char msm[];
 	bf16 *A = reinterpret_cast<bf16 *>(msm);
@@ -140,70 +132,16 @@ mlp_forward_kernel(const bf16 *__restrict__ X, long long n, MlpWeights w, float 
 			*reinterpret_cast<uint4 *>(B + (wr + rr) * kActStride + c8 * 8) = v;
 		}
 		__syncwarp();
-		dense<kInP, kHid, 0, TRAIN>(B, A, w.wt1, w.b1, wr, r0, n, nullptr, P1, H1);
+		dense<kInP, kHid, 0>(B, A, w.wt1, w.b1, wr, r0, n, nullptr);
 		__syncwarp();
-		dense<kHid, kHid, 0, TRAIN>(A, B, w.wt2, w.b2, wr, r0, n, nullptr, P2, H2);
+		dense<kHid, kHid, 0>(A, B, w.wt2, w.b2, wr, r0, n, nullptr);
 		__syncwarp();
-		dense<kHid, kOut, 1, TRAIN>(B, nullptr, w.wt3, w.b3, wr, r0, n, out, nullptr, nullptr);
+		dense<kHid, kOut, 1>(B, nullptr, w.wt3, w.b3, wr, r0, n, out);
 		__syncwarp();
 	}
 }
 
 constexpr size_t kForwardSmem = sizeof(bf16) * 2 * kRowsPerCta * kActStride;
-
-// C[m][n] = sum_k A(m,k) B(k,n) with A(m,k) = a[m*am + k*ak], B(k,n) = b[k*bk + n*bn],
-// bf16 operands, float result (ldc).  64 x 64 tiles, k in steps of 32.
-__global__ void __launch_bounds__(128)
-gemm_bf16_kernel(const bf16 *__restrict__ a, long long am, long long ak, const bf16 *__restrict__ b,
-                 long long bk, long long bn, float *__restrict__ c, int ldc, int M, int N, long long K)
-{
-	constexpr int S = 40;   // bf16 pitch of the k-major shared tiles
-	__shared__ __align__(16) bf16 As[64 * S];
-	__shared__ __align__(16) bf16 Bs[64 * S];
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-	const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-	float acc[8][4];
-#pragma unroll
-	for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-	const bf16 zero = __float2bfloat16_rn(0.f);
-	for (long long k0 = 0; k0 < K; k0 += 32) {
-		__syncthreads();
-		for (int i = tid; i < 64 * 32; i += 128) {
-			// consecutive threads along whichever index has unit stride
-			int r, kk;
-			if (ak == 1) { r = i / 32; kk = i % 32; } else { r = i % 64; kk = i / 64; }
-			const long long m = m0 + r, k = k0 + kk;
-			As[r * S + kk] = (m < M && k < K) ? a[m * am + k * ak] : zero;
-			int q, kb;
-			if (bk == 1) { q = i / 32; kb = i % 32; } else { q = i % 64; kb = i / 64; }
-			const long long nn = n0 + q, k2 = k0 + kb;
-			Bs[q * S + kb] = (nn < N && k2 < K) ? b[k2 * bk + nn * bn] : zero;
-		}
-		__syncthreads();
-#pragma unroll
-		for (int ks = 0; ks < 32; ks += 16) {
-			uint32_t af[4];
-			af[0] = ld_u32(As + (warp * 16 + g) * S + ks + 2 * t);
-			af[1] = ld_u32(As + (warp * 16 + g + 8) * S + ks + 2 * t);
-			af[2] = ld_u32(As + (warp * 16 + g) * S + ks + 8 + 2 * t);
-			af[3] = ld_u32(As + (warp * 16 + g + 8) * S + ks + 8 + 2 * t);
-#pragma unroll
-			for (int j = 0; j < 8; j++)
-				mma_bf16(acc[j], af, ld_u32(Bs + (j * 8 + g) * S + ks + 2 * t),
-				         ld_u32(Bs + (j * 8 + g) * S + ks + 8 + 2 * t));
-		}
-	}
-#pragma unroll
-	for (int j = 0; j < 8; j++)
-#pragma unroll
-		for (int h = 0; h < 2; h++) {
-			const int m = m0 + warp * 16 + g + 8 * h;
-			const int nn = n0 + j * 8 + 2 * t;
-			if (m >= M) continue;
-			if (nn < N) c[(long long)m * ldc + nn] = acc[j][2 * h];
-			if (nn + 1 < N) c[(long long)m * ldc + nn + 1] = acc[j][2 * h + 1];
-		}
-}
 
 // float features [n][65] -> bf16 [n][80] (zero padded)
 __global__ void pack_features_kernel(const float *__restrict__ f, long long n, bf16 *__restrict__ X)
@@ -216,97 +154,381 @@ __global__ void pack_features_kernel(const float *__restrict__ f, long long n, b
 	}
 }
 
-// master (float, W[in][out]) -> transposed bf16 working copy
-__global__ void pack_weights_kernel(const float *__restrict__ m, bf16 *__restrict__ wt)
+// ---------------------------------------------------------------------------
+// Training.  One step is three launches:
+//   train_rows_kernel   forward and backward of 32 rows per CTA, all layers; the
+//                       pre-activations stay in registers (a warp's columns are
+//                       the same in the forward and the backward pass of a
+//                       layer); leaves the BF16 activations and gradients of
+//                       every layer, and per-CTA sums for the biases and the loss
+//   weight_grad_kernel  the three products activations^T . gradients, 64 x 64
+//                       tiles, the rows split over CTAs
+//   update_kernel       the splits summed in a fixed order (no atomics: a step is
+//                       reproducible), AdamW, and the weights' BF16 copies
+// Separate kernels per layer with 16 CTAs walking all 8192 rows took 5.6 ms for
+// a step of 8192 rows; these take 32 + 12 + 10 us.  What bounds them: the latency
+// of one wave of CTAs (4.8 GFLOP are 3 us of the tensor cores' time), the
+// weights' trip through L2 to every CTA, and erff.
+//
+// Weights as B operands of mma.m16n8k16, in fragment order: for a tile of 8
+// outputs and a pair of k-steps, lane (g = lane / 4, t = lane % 4) holds
+// k = 2t, 2t+1, 2t+8, 2t+9 of output g of both steps in 16 bytes.
+// ---------------------------------------------------------------------------
+constexpr int kTrainRows = 32, kTrainThreads = 512;   // rows and threads per CTA of train_rows_kernel
+constexpr int kGradTile = 64, kMaxSplits = 16, kSplitRows = 512;
+constexpr int kInF = 96;                 // inputs padded to whole pairs of k-steps
+constexpr int kFragF1 = 0, kFragF2 = kFragF1 + kInF * kHid, kFragF3 = kFragF2 + kHid * kHid,
+              kFragB3 = kFragF3 + kHid * kOut, kFragB2 = kFragB3 + kOut * kHid, kFragSize = kFragB2 + kHid * kHid;
+constexpr int kBiases = kHid + kHid + kOut;
+
+// Place of B(k, n) in a fragment-ordered operand of K rows.
+__host__ __device__ __forceinline__ int frag_at(int k, int n, int K)
 {
-	const int n1 = kHid * kInP, n2 = kHid * kHid, n3 = kOut * kHid;
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2 + n3; i += gridDim.x * blockDim.x) {
-		float v;
-		if (i < n1) {
-			const int o = i / kInP, k = i % kInP;
-			v = m[kMlpOffW1 + k * kHid + o];
-		} else if (i < n1 + n2) {
-			const int j = i - n1, o = j / kHid, k = j % kHid;
-			v = m[kMlpOffW2 + k * kHid + o];
-		} else {
-			const int j = i - n1 - n2, o = j / kHid, k = j % kHid;
-			v = m[kMlpOffW3 + k * kOut + o];
-		}
-		wt[i] = __float2bfloat16_rn(v);
+	const int pair = k >> 5, ks = k >> 4 & 1, kk = k & 15;
+	const int t = (kk & 7) >> 1, half = kk >> 3, lane = (n & 7) * 4 + t;
+	return (((n >> 3) * (K >> 5) + pair) * 32 + lane) * 8 + ks * 4 + half * 2 + (kk & 1);
+}
+
+// acc[mi][j] = A (MI x 16 rows, K columns, shared, pitch ldA) . B tiles tile0 + j
+template <int K, int MI, int NT>
+__device__ __forceinline__ void rows_mma(const bf16 *A, int ldA, const bf16 *__restrict__ B, int tile0,
+                                         float (&acc)[MI][NT][4])
+{
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+	for (int mi = 0; mi < MI; mi++)
+#pragma unroll
+		for (int j = 0; j < NT; j++) acc[mi][j][0] = acc[mi][j][1] = acc[mi][j][2] = acc[mi][j][3] = 0.f;
+#pragma unroll 4
+	for (int p = 0; p < K / 32; p++) {
+		uint4 b[NT];
+#pragma unroll
+		for (int j = 0; j < NT; j++)
+			b[j] = __ldg(reinterpret_cast<const uint4 *>(B) + ((size_t)(tile0 + j) * (K / 32) + p) * 32 + lane);
+#pragma unroll
+		for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+			for (int mi = 0; mi < MI; mi++) {
+				const bf16 *r = A + (mi * 16 + g) * ldA + p * 32 + ks * 16 + 2 * t;
+				const uint32_t a[4] = {ld_u32(r), ld_u32(r + 8 * ldA), ld_u32(r + 8), ld_u32(r + 8 * ldA + 8)};
+#pragma unroll
+				for (int j = 0; j < NT; j++) mma_bf16(acc[mi][j], a, ks ? b[j].z : b[j].x, ks ? b[j].w : b[j].y);
+			}
 	}
 }
 
-// dL/dz3 of the mean squared error through the sigmoid, and per-block loss sums
-__global__ void out_grad_kernel(const float *__restrict__ y, const float *__restrict__ tgt, long long n,
-                                float *__restrict__ dP, bf16 *__restrict__ dPb, float *__restrict__ partial)
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b)
 {
-	__shared__ float red[256];
-	const float scale = 2.f / (float)(n * kOut);
-	float s = 0.f;
-	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * kOut;
-	     i += (long long)gridDim.x * blockDim.x) {
-		const float e = y[i] - tgt[i];
-		s += e * e;
-		const float d = scale * e * y[i] * (1.f - y[i]);
-		dP[i] = d;
-		dPb[i] = __float2bfloat16_rn(d);
+	__nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+	return *reinterpret_cast<uint32_t *>(&v);
+}
+
+// Sum of a column's values over the lanes that hold its rows (g = 0 .. 7).
+__device__ __forceinline__ float column_sum(float v)
+{
+	v += __shfl_xor_sync(0xffffffffu, v, 4);
+	v += __shfl_xor_sync(0xffffffffu, v, 8);
+	v += __shfl_xor_sync(0xffffffffu, v, 16);
+	return v;
+}
+
+struct TrainRows {
+	const float *feat, *target;
+	long long n;
+	const bf16 *frag;
+	const float *master;
+	bf16 *X, *H1, *H2, *D1, *D2, *D3;   // [rows][96], [rows][256] x 2, then the gradients
+	float *bias_part, *loss_part;       // [CTAs][kBiases], [CTAs]
+};
+
+__global__ void __launch_bounds__(kTrainThreads, 2)
+train_rows_kernel(TrainRows a)
+{
+	constexpr int XP = kInF + 8, HP = kHid + 8, OP = kOut + 8;   // pitches without bank conflicts
+	__shared__ __align__(16) bf16 Xs[kTrainRows * XP], Hs[kTrainRows * HP], Gs[kTrainRows * HP], Ds[kTrainRows * OP];
+	__shared__ float s_loss[kTrainThreads / 32], s_db3[2][kOut];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+	const long long r0 = (long long)blockIdx.x * kTrainRows;
+	for (int i = tid; i < kTrainRows * kInF; i += kTrainThreads) {
+		const int r = i / kInF, c = i % kInF;
+		const bf16 v = __float2bfloat16_rn(c < kIn && r0 + r < a.n ? a.feat[(r0 + r) * kIn + c] : 0.f);
+		Xs[r * XP + c] = v;
+		a.X[(r0 + r) * kInF + c] = v;
 	}
-	red[threadIdx.x] = s;
 	__syncthreads();
-	for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-		if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+	const int c0 = warp * 16;            // this warp's columns of the hidden layers
+	float p1[2][2][4], p2[2][2][4];
+	// hidden layer: pre-activations to p, activations to shared memory and H
+	auto hidden = [&](float (&p)[2][2][4], const float *bias, bf16 *out, bf16 *H) {
+#pragma unroll
+		for (int j = 0; j < 2; j++) {
+			const int c = c0 + j * 8 + 2 * t;
+			const float b0 = __ldg(bias + c), b1 = __ldg(bias + c + 1);
+#pragma unroll
+			for (int mi = 0; mi < 2; mi++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					const int r = mi * 16 + g + 8 * h;
+					p[mi][j][2 * h] += b0;
+					p[mi][j][2 * h + 1] += b1;
+					const uint32_t v = pack_bf16(gelu(p[mi][j][2 * h]), gelu(p[mi][j][2 * h + 1]));
+					*reinterpret_cast<uint32_t *>(out + r * HP + c) = v;
+					*reinterpret_cast<uint32_t *>(H + (r0 + r) * kHid + c) = v;
+				}
+		}
+	};
+	rows_mma<kInF, 2, 2>(Xs, XP, a.frag + kFragF1, warp * 2, p1);
+	hidden(p1, a.master + kMlpOffB1, Hs, a.H1);
+	__syncthreads();
+	rows_mma<kHid, 2, 2>(Hs, HP, a.frag + kFragF2, warp * 2, p2);
+	hidden(p2, a.master + kMlpOffB2, Gs, a.H2);
+	__syncthreads();
+	float *bias_part = a.bias_part + (size_t)blockIdx.x * kBiases;
+	{
+		// output layer: sigmoid, squared error, its gradient; a warp takes 8 columns
+		// of 16 rows
+		const int m0 = (warp >> 3) * 16;
+		float o[1][1][4];
+		rows_mma<kHid, 1, 1>(Gs + m0 * HP, HP, a.frag + kFragF3, warp & 7, o);
+		const int c = (warp & 7) * 8 + 2 * t;
+		const float b0 = __ldg(a.master + kMlpOffB3 + c), b1 = __ldg(a.master + kMlpOffB3 + c + 1);
+		const float scale = 2.f / (float)(a.n * kOut);
+		float loss = 0.f, s0 = 0.f, s1 = 0.f;
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const int r = m0 + g + 8 * h;
+			float d[2] = {0.f, 0.f};
+			if (r0 + r < a.n) {
+				const float *tg = a.target + (r0 + r) * kOut + c;
+#pragma unroll
+				for (int q = 0; q < 2; q++) {
+					const float y = 1.f / (1.f + expf(-(o[0][0][2 * h + q] + (q ? b1 : b0))));
+					const float e = y - tg[q];
+					loss += e * e;
+					d[q] = scale * e * y * (1.f - y);
+				}
+			}
+			s0 += d[0];
+			s1 += d[1];
+			const uint32_t v = pack_bf16(d[0], d[1]);
+			*reinterpret_cast<uint32_t *>(Ds + r * OP + c) = v;
+			*reinterpret_cast<uint32_t *>(a.D3 + (r0 + r) * kOut + c) = v;
+		}
+		s0 = column_sum(s0);
+		s1 = column_sum(s1);
+		if (g == 0) { s_db3[warp >> 3][c] = s0; s_db3[warp >> 3][c + 1] = s1; }
+#pragma unroll
+		for (int s = 16; s > 0; s >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, s);
+		if (lane == 0) s_loss[warp] = loss;
+	}
+	__syncthreads();
+	if (tid < kOut) bias_part[2 * kHid + tid] = s_db3[0][tid] + s_db3[1][tid];
+	if (tid == 0) {
+		float l = 0.f;
+		for (int i = 0; i < kTrainThreads / 32; i++) l += s_loss[i];
+		a.loss_part[blockIdx.x] = l;
+	}
+	// gradient of a hidden layer: d = (dH) GELU'(p), to shared memory (when another
+	// layer follows) and D, its column sums to the bias
+	auto back = [&](const float (&dh)[2][2][4], const float (&p)[2][2][4], bf16 *out, bf16 *D, float *db) {
+#pragma unroll
+		for (int j = 0; j < 2; j++) {
+			const int c = c0 + j * 8 + 2 * t;
+			float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+			for (int mi = 0; mi < 2; mi++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					const int r = mi * 16 + g + 8 * h;
+					const float d0 = dh[mi][j][2 * h] * gelu_grad(p[mi][j][2 * h]);
+					const float d1 = dh[mi][j][2 * h + 1] * gelu_grad(p[mi][j][2 * h + 1]);
+					s0 += d0;
+					s1 += d1;
+					const uint32_t v = pack_bf16(d0, d1);
+					if (out) *reinterpret_cast<uint32_t *>(out + r * HP + c) = v;
+					*reinterpret_cast<uint32_t *>(D + (r0 + r) * kHid + c) = v;
+				}
+			s0 = column_sum(s0);
+			s1 = column_sum(s1);
+			if (g == 0) { db[c] = s0; db[c + 1] = s1; }
+		}
+	};
+	float dh[2][2][4];
+	rows_mma<kOut, 2, 2>(Ds, OP, a.frag + kFragB3, warp * 2, dh);
+	back(dh, p2, Hs, a.D2, bias_part + kHid);     // Hs is free: layer 2 has read it
+	__syncthreads();
+	rows_mma<kHid, 2, 2>(Hs, HP, a.frag + kFragB2, warp * 2, dh);
+	back(dh, p1, nullptr, a.D1, bias_part);
+}
+
+__device__ __forceinline__ void ldmatrix_t(uint32_t (&r)[4], const bf16 *p)
+{
+	const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+	             : "r"(s)
+	             : "memory");
+}
+
+// part[split][offset ..] = A^T . B over the split's rows, one 64 x 64 tile per CTA:
+// layer 2 (16 tiles), layer 3 (4), layer 1 (8, its last rows cut off at 80).
+__global__ void __launch_bounds__(128)
+weight_grad_kernel(const bf16 *__restrict__ X, const bf16 *__restrict__ H1, const bf16 *__restrict__ H2,
+                   const bf16 *__restrict__ D1, const bf16 *__restrict__ D2, const bf16 *__restrict__ D3, int rows,
+                   int split_rows, float *__restrict__ part)
+{
+	constexpr int KB = 32, SP = kGradTile + 8;
+	__shared__ __align__(16) bf16 As[2][KB * SP], Bs[2][KB * SP];
+	const int tile = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+	const bf16 *A, *B;
+	int lda, ldb, m0, n0, M, N, off;
+	if (tile < 16) { A = H1; B = D2; lda = ldb = kHid; m0 = tile / 4 * 64; n0 = tile % 4 * 64; M = N = kHid; off = kMlpOffW2; }
+	else if (tile < 20) { A = H2; B = D3; lda = kHid; ldb = kOut; m0 = (tile - 16) * 64; n0 = 0; M = kHid; N = kOut; off = kMlpOffW3; }
+	else { A = X; B = D1; lda = kInF; ldb = kHid; m0 = (tile - 20) / 4 * 64; n0 = (tile - 20) % 4 * 64; M = kInP; N = kHid; off = kMlpOffW1; }
+	const int k0 = blockIdx.y * split_rows, k1 = min(rows, k0 + split_rows);
+	// a 32 x 64 block of an operand: 256 pieces of 16 bytes, two per thread; columns
+	// past the operand's width (layer 1's second tile) stay zero
+	auto load = [&](bf16 *s, const bf16 *p, int ld, int c0, int r0) {
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const int i = tid + h * 128, r = i >> 3, c = (i & 7) * 8;
+			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s + r * SP + c);
+			const bool in = c0 + c < ld;
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(p + (size_t)(r0 + r) * ld + (in ? c0 + c : 0)),
+			             "r"(in ? 16 : 0));
+		}
+	};
+	float acc[8][4];
+#pragma unroll
+	for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+	int buf = 0;
+	if (k0 < k1) {
+		load(As[0], A, lda, m0, k0);
+		load(Bs[0], B, ldb, n0, k0);
+	}
+	asm volatile("cp.async.commit_group;\n");
+	for (int k = k0; k < k1; k += KB, buf ^= 1) {
+		if (k + KB < k1) {
+			load(As[buf ^ 1], A, lda, m0, k + KB);
+			load(Bs[buf ^ 1], B, ldb, n0, k + KB);
+		}
+		asm volatile("cp.async.commit_group;\n");
+		asm volatile("cp.async.wait_group 1;\n");
+		__syncthreads();
+		// rows are the summed index: both operands come out of shared memory
+		// transposed
+#pragma unroll
+		for (int ks = 0; ks < KB; ks += 16) {
+			uint32_t af[4];
+			// 8 x 8 blocks (k, m): (0, 0), (0, 8), (8, 0), (8, 8)
+			ldmatrix_t(af, As[buf] + (ks + (lane >> 4) * 8 + (lane & 7)) * SP + warp * 16 + (lane >> 3 & 1) * 8);
+#pragma unroll
+			for (int j = 0; j < 8; j += 2) {
+				uint32_t bq[4];
+				// blocks (k, n): (0, 0), (8, 0), (0, 8), (8, 8)
+				ldmatrix_t(bq, Bs[buf] + (ks + (lane >> 3 & 1) * 8 + (lane & 7)) * SP + j * 8 + (lane >> 4) * 8);
+				mma_bf16(acc[j], af, bq[0], bq[1]);
+				mma_bf16(acc[j + 1], af, bq[2], bq[3]);
+			}
+		}
 		__syncthreads();
 	}
-	if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
+	float *out = part + (size_t)blockIdx.y * kMlpMasterSize + off;
+#pragma unroll
+	for (int j = 0; j < 8; j++)
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const int m = m0 + warp * 16 + g + 8 * h, c = n0 + j * 8 + 2 * t;
+			if (m < M && c < N)
+				*reinterpret_cast<float2 *>(out + (size_t)m * N + c) = make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+		}
 }
 
-// dP = dH * GELU'(P)
-__global__ void gelu_back_kernel(const float *__restrict__ dH, const float *__restrict__ P, long long cnt,
-                                 float *__restrict__ dP, bf16 *__restrict__ dPb)
+// The weight's BF16 copies: the transposed one of the inference kernel and the
+// fragment-ordered ones (frag may be null).
+__device__ __forceinline__ void store_weight(int i, float v, bf16 *wt, bf16 *frag)
 {
-	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt;
-	     i += (long long)gridDim.x * blockDim.x) {
-		const float d = dH[i] * gelu_grad(P[i]);
-		dP[i] = d;
-		dPb[i] = __float2bfloat16_rn(d);
+	const bf16 b = __float2bfloat16_rn(v);
+	if (i < kMlpOffB1) {
+		const int k = i / kHid, o = i % kHid;
+		wt[o * kInP + k] = b;
+		if (frag) frag[kFragF1 + frag_at(k, o, kInF)] = b;
+	} else if (i >= kMlpOffW2 && i < kMlpOffB2) {
+		const int j = i - kMlpOffW2, k = j / kHid, o = j % kHid;
+		wt[kHid * kInP + o * kHid + k] = b;
+		if (frag) {
+			frag[kFragF2 + frag_at(k, o, kHid)] = b;
+			frag[kFragB2 + frag_at(o, k, kHid)] = b;
+		}
+	} else if (i >= kMlpOffW3 && i < kMlpOffB3) {
+		const int j = i - kMlpOffW3, k = j / kOut, o = j % kOut;
+		wt[kHid * kInP + kHid * kHid + o * kHid + k] = b;
+		if (frag) {
+			frag[kFragF3 + frag_at(k, o, kHid)] = b;
+			frag[kFragB3 + frag_at(o, k, kOut)] = b;
+		}
 	}
 }
 
-// bias gradient: column sums of dP [n][N] (one thread per column, fixed order)
-__global__ void colsum_kernel(const float *__restrict__ dP, long long n, int N, float *__restrict__ out)
+__global__ void pack_weights_kernel(const float *__restrict__ m, bf16 *__restrict__ wt, bf16 *__restrict__ frag)
 {
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c >= N) return;
-	float s = 0.f;
-	for (long long r = 0; r < n; r++) s += dP[r * N + c];
-	out[c] = s;
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpMasterSize; i += gridDim.x * blockDim.x)
+		store_weight(i, m[i], wt, frag);
 }
 
-__global__ void sum_kernel(const float *__restrict__ part, int n, float *__restrict__ out)
+__device__ __forceinline__ bool is_bias(int i)
 {
-	if (threadIdx.x == 0 && blockIdx.x == 0) {
+	return (i >= kMlpOffB1 && i < kMlpOffW2) || (i >= kMlpOffB2 && i < kMlpOffW3) || i >= kMlpOffB3;
+}
+
+struct Update {
+	const float *part, *bias_part, *loss_part;
+	int splits, ctas;
+	float *grad, *loss;                  // grad: written when step is 0
+	int step;
+	float *p, *m, *v;
+	float lr, b1, b2, eps, wd, c1, c2;
+	bf16 *wt, *frag;
+};
+
+// Sums of the splits (weights: a thread each; biases and the loss: a warp each),
+// then AdamW; weight decay on the matrices, not the biases.
+__global__ void __launch_bounds__(256)
+update_kernel(Update u)
+{
+	auto apply = [&](int i, float g) {
+		if (!u.step) {
+			u.grad[i] = g;
+			return;
+		}
+		const float mi = u.b1 * u.m[i] + (1.f - u.b1) * g;
+		const float vi = u.b2 * u.v[i] + (1.f - u.b2) * g * g;
+		u.m[i] = mi;
+		u.v[i] = vi;
+		float q = u.p[i];
+		const bool bias = is_bias(i);
+		if (!bias) q -= u.lr * u.wd * q;
+		q -= u.lr * (mi / u.c1) / (sqrtf(vi / u.c2) + u.eps);
+		u.p[i] = q;
+		if (!bias) store_weight(i, q, u.wt, u.frag);
+	};
+	const int nthreads = gridDim.x * blockDim.x, id = blockIdx.x * blockDim.x + threadIdx.x;
+	for (int i = id; i < kMlpMasterSize; i += nthreads) {
+		if (is_bias(i)) continue;
+		float g = 0.f;
+#pragma unroll 4
+		for (int s = 0; s < u.splits; s++) g += u.part[(size_t)s * kMlpMasterSize + i];
+		apply(i, g);
+	}
+	const int lane = threadIdx.x & 31;
+	for (int b = id >> 5; b <= kBiases; b += nthreads >> 5) {
 		double s = 0.0;
-		for (int i = 0; i < n; i++) s += part[i];
-		*out = (float)s;
-	}
-}
-
-// AdamW on the master weights; weight decay on the matrices, not the biases
-__global__ void adamw_kernel(float *__restrict__ p, const float *__restrict__ gr, float *__restrict__ m,
-                             float *__restrict__ v, int n, float lr, float b1, float b2, float eps, float wd,
-                             float c1, float c2)
-{
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		const bool bias = (i >= kMlpOffB1 && i < kMlpOffW2) || (i >= kMlpOffB2 && i < kMlpOffW3) || i >= kMlpOffB3;
-		const float g = gr[i];
-		const float mi = b1 * m[i] + (1.f - b1) * g;
-		const float vi = b2 * v[i] + (1.f - b2) * g * g;
-		m[i] = mi;
-		v[i] = vi;
-		float q = p[i];
-		if (!bias) q -= lr * wd * q;
-		q -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-		p[i] = q;
+		for (int c = lane; c < u.ctas; c += 32) s += b < kBiases ? u.bias_part[(size_t)c * kBiases + b] : u.loss_part[c];
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		if (lane != 0) continue;
+		if (b == kBiases) *u.loss = (float)s;
+		else apply(b < kHid ? kMlpOffB1 + b : b < 2 * kHid ? kMlpOffB2 + b - kHid : kMlpOffB3 + b - 2 * kHid, (float)s);
 	}
 }
 
@@ -322,19 +544,18 @@ cudaError_t launch_mlp_forward(const uint16_t *X, long long n, const MlpWeights 
                                cudaStream_t st)
 {
 	if (n <= 0) return cudaSuccess;
-	cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                     (int)kForwardSmem);
 	if (e != cudaSuccess) return e;
 	const long long need = (n + kRowsPerCta - 1) / kRowsPerCta;
 	const int nb = (int)std::min<long long>(need, (long long)nsm * 3);
-	mlp_forward_kernel<false><<<nb, 128, kForwardSmem, st>>>(reinterpret_cast<const bf16 *>(X), n, w, out,
-	                                                         nullptr, nullptr, nullptr, nullptr);
+	mlp_forward_kernel<<<nb, 128, kForwardSmem, st>>>(reinterpret_cast<const bf16 *>(X), n, w, out);
 	return cudaGetLastError();
 }
 
 cudaError_t launch_pack_weights(const float *master, uint16_t *wt, cudaStream_t st)
 {
-	pack_weights_kernel<<<256, 256, 0, st>>>(master, reinterpret_cast<bf16 *>(wt));
+	pack_weights_kernel<<<256, 256, 0, st>>>(master, reinterpret_cast<bf16 *>(wt), nullptr);
 	return cudaGetLastError();
 }
 
@@ -380,10 +601,10 @@ struct bm4dof_trainer {
 	cudaStream_t st = nullptr;
 	float *master = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
 	uint16_t *wt = nullptr;
-	// activations of one batch
-	bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dPb = nullptr;
-	float *P1 = nullptr, *P2 = nullptr, *Y = nullptr, *dP = nullptr, *dH = nullptr, *part = nullptr,
-	      *loss = nullptr;
+	bf16 *frag = nullptr;        // the weights in fragment order
+	// activations and gradients of one batch (rows padded to whole CTAs)
+	bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *D1 = nullptr, *D2 = nullptr, *D3 = nullptr;
+	float *part = nullptr, *bias_part = nullptr, *loss_part = nullptr, *loss = nullptr;
 };
 
 namespace {
@@ -397,52 +618,62 @@ namespace {
 		}                                                                                    \
 	} while (0)
 
-constexpr int kPartBlocks = 512;
-
 void free_trainer(bm4dof_trainer *t)
 {
-	void *ps[] = {t->master, t->grad, t->m1, t->m2, t->wt, t->X, t->H1, t->H2, t->dPb,
-	              t->P1, t->P2, t->Y, t->dP, t->dH, t->part, t->loss};
+	void *ps[] = {t->master, t->grad, t->m1, t->m2, t->wt, t->frag, t->X, t->H1, t->H2, t->D1, t->D2, t->D3,
+	              t->part, t->bias_part, t->loss_part, t->loss};
 	for (void *p : ps)
 		if (p) cudaFree(p);
 	if (t->st) cudaStreamDestroy(t->st);
 	delete t;
 }
 
-// forward + backward of n rows (n <= batch): gradients into t->grad, loss into t->loss
-bm4dof_status forward_backward(bm4dof_trainer *t, const float *feat, const float *target, long long n)
+// forward + backward of n rows (n <= batch), then the gradients into t->grad
+// (u.step 0) or an AdamW step; the loss into t->loss
+bm4dof_status train_batch(bm4dof_trainer *t, const float *feat, const float *target, long long n, Update u)
 {
 	cudaStream_t st = t->st;
-	const MlpWeights w = mlp_weights(t->wt, t->master);
-	pack_features_kernel<<<blocks_for(n * kInP, 256), 256, 0, st>>>(feat, n, t->X);
-	TCK(cudaFuncSetAttribute(mlp_forward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                         (int)kForwardSmem));
-	const int nb = (int)std::min<long long>((n + kRowsPerCta - 1) / kRowsPerCta, (long long)t->nsm * 3);
-	mlp_forward_kernel<true><<<nb, 128, kForwardSmem, st>>>(t->X, n, w, t->Y, t->P1, t->H1, t->P2, t->H2);
-	out_grad_kernel<<<kPartBlocks, 256, 0, st>>>(t->Y, target, n, t->dP, t->dPb, t->part);
-	sum_kernel<<<1, 32, 0, st>>>(t->part, kPartBlocks, t->loss);
-	const bf16 *wt = reinterpret_cast<const bf16 *>(t->wt);
-	const bf16 *wt2 = wt + kHid * kInP, *wt3 = wt2 + kHid * kHid;
-	auto gemm = [&](const bf16 *a, long long am, long long ak, const bf16 *b, long long bk, long long bn,
-	                float *c, int ldc, int M, int N, long long K) {
-		dim3 grid((N + 63) / 64, (M + 63) / 64);
-		gemm_bf16_kernel<<<grid, 128, 0, st>>>(a, am, ak, b, bk, bn, c, ldc, M, N, K);
-	};
-	// layer 3: dW3[i][j] = sum_b H2[b][i] dP3[b][j]; db3; dH2 = dP3 . W3^T
-	gemm(t->H2, 1, kHid, t->dPb, kOut, 1, t->grad + kMlpOffW3, kOut, kHid, kOut, n);
-	colsum_kernel<<<1, kOut, 0, st>>>(t->dP, n, kOut, t->grad + kMlpOffB3);
-	gemm(t->dPb, kOut, 1, wt3, kHid, 1, t->dH, kHid, (int)n, kHid, kOut);
-	gelu_back_kernel<<<blocks_for(n * kHid, 256), 256, 0, st>>>(t->dH, t->P2, n * kHid, t->dP, t->dPb);
-	// layer 2
-	gemm(t->H1, 1, kHid, t->dPb, kHid, 1, t->grad + kMlpOffW2, kHid, kHid, kHid, n);
-	colsum_kernel<<<1, kHid, 0, st>>>(t->dP, n, kHid, t->grad + kMlpOffB2);
-	gemm(t->dPb, kHid, 1, wt2, kHid, 1, t->dH, kHid, (int)n, kHid, kHid);
-	gelu_back_kernel<<<blocks_for(n * kHid, 256), 256, 0, st>>>(t->dH, t->P1, n * kHid, t->dP, t->dPb);
-	// layer 1 (rows 65..79 of dW1 come out zero: their inputs are zero)
-	gemm(t->X, 1, kInP, t->dPb, kHid, 1, t->grad + kMlpOffW1, kHid, kInP, kHid, n);
-	colsum_kernel<<<1, kHid, 0, st>>>(t->dP, n, kHid, t->grad + kMlpOffB1);
+	const int ctas = (int)((n + kTrainRows - 1) / kTrainRows), rows = ctas * kTrainRows;
+	TrainRows a;
+	a.feat = feat;
+	a.target = target;
+	a.n = n;
+	a.frag = t->frag;
+	a.master = t->master;
+	a.X = t->X;
+	a.H1 = t->H1;
+	a.H2 = t->H2;
+	a.D1 = t->D1;
+	a.D2 = t->D2;
+	a.D3 = t->D3;
+	a.bias_part = t->bias_part;
+	a.loss_part = t->loss_part;
+	train_rows_kernel<<<ctas, kTrainThreads, 0, st>>>(a);
+	// rows split into pieces of at least kSplitRows, whole 32-row blocks each
+	const int want = std::max(1, std::min(kMaxSplits, (rows + kSplitRows - 1) / kSplitRows));
+	const int split_rows = ((rows + want - 1) / want + 31) / 32 * 32, splits = (rows + split_rows - 1) / split_rows;
+	weight_grad_kernel<<<dim3(28, splits), 128, 0, st>>>(t->X, t->H1, t->H2, t->D1, t->D2, t->D3, rows, split_rows, t->part);
+	u.part = t->part;
+	u.bias_part = t->bias_part;
+	u.loss_part = t->loss_part;
+	u.splits = splits;
+	u.ctas = ctas;
+	u.grad = t->grad;
+	u.loss = t->loss;
+	u.p = t->master;
+	u.m = t->m1;
+	u.v = t->m2;
+	u.wt = reinterpret_cast<bf16 *>(t->wt);
+	u.frag = t->frag;
+	update_kernel<<<blocks_for(kMlpMasterSize, 256), 256, 0, st>>>(u);
 	TCK(cudaGetLastError());
 	return BM4DOF_OK;
+}
+
+cudaError_t pack_trainer(bm4dof_trainer *t)
+{
+	pack_weights_kernel<<<256, 256, 0, t->st>>>(t->master, reinterpret_cast<bf16 *>(t->wt), t->frag);
+	return cudaGetLastError();
 }
 
 bool trainer_ok(bm4dof_trainer *t, const void *feat, const void *target, unsigned n)
@@ -475,23 +706,23 @@ bm4dof_status bm4dof_trainer_create(bm4dof_trainer **out, int device, unsigned b
 	t->device = device;
 	t->batch = batch;
 	cudaDeviceGetAttribute(&t->nsm, cudaDevAttrMultiProcessorCount, device);
-	const size_t B = batch;
+	const size_t ctas = ((size_t)batch + kTrainRows - 1) / kTrainRows, B = ctas * kTrainRows;
 	bool ok = cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking) == cudaSuccess &&
 	          cudaMalloc(&t->master, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->grad, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->m1, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->m2, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->wt, sizeof(uint16_t) * kMlpWtSize) == cudaSuccess &&
-	          cudaMalloc(&t->X, sizeof(bf16) * B * kInP) == cudaSuccess &&
+	          cudaMalloc(&t->frag, sizeof(bf16) * kFragSize) == cudaSuccess &&
+	          cudaMalloc(&t->X, sizeof(bf16) * B * kInF) == cudaSuccess &&
 	          cudaMalloc(&t->H1, sizeof(bf16) * B * kHid) == cudaSuccess &&
 	          cudaMalloc(&t->H2, sizeof(bf16) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->dPb, sizeof(bf16) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->P1, sizeof(float) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->P2, sizeof(float) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->Y, sizeof(float) * B * kOut) == cudaSuccess &&
-	          cudaMalloc(&t->dP, sizeof(float) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->dH, sizeof(float) * B * kHid) == cudaSuccess &&
-	          cudaMalloc(&t->part, sizeof(float) * kPartBlocks) == cudaSuccess &&
+	          cudaMalloc(&t->D1, sizeof(bf16) * B * kHid) == cudaSuccess &&
+	          cudaMalloc(&t->D2, sizeof(bf16) * B * kHid) == cudaSuccess &&
+	          cudaMalloc(&t->D3, sizeof(bf16) * B * kOut) == cudaSuccess &&
+	          cudaMalloc(&t->part, sizeof(float) * kMaxSplits * kMlpMasterSize) == cudaSuccess &&
+	          cudaMalloc(&t->bias_part, sizeof(float) * ctas * kBiases) == cudaSuccess &&
+	          cudaMalloc(&t->loss_part, sizeof(float) * ctas) == cudaSuccess &&
 	          cudaMalloc(&t->loss, sizeof(float)) == cudaSuccess;
 	if (!ok) {
 		cudaGetLastError();
@@ -519,7 +750,8 @@ bm4dof_status bm4dof_trainer_create(bm4dof_trainer **out, int device, unsigned b
 	TCK(cudaMemsetAsync(t->m1, 0, sizeof(float) * kMlpMasterSize, t->st));
 	TCK(cudaMemsetAsync(t->m2, 0, sizeof(float) * kMlpMasterSize, t->st));
 	TCK(cudaMemsetAsync(t->grad, 0, sizeof(float) * kMlpMasterSize, t->st));
-	TCK(launch_pack_weights(t->master, t->wt, t->st));
+	TCK(cudaMemsetAsync(t->frag, 0, sizeof(bf16) * kFragSize, t->st));   // inputs 80..95 stay zero
+	TCK(pack_trainer(t));
 	TCK(cudaStreamSynchronize(t->st));
 	*out = t;
 	return BM4DOF_OK;
@@ -553,7 +785,7 @@ bm4dof_status bm4dof_trainer_params(bm4dof_trainer *t, float *params, size_t n, 
 	if (set) {
 		mlp_public_to_master(params, master.data());
 		TCK(cudaMemcpyAsync(t->master, master.data(), sizeof(float) * kMlpMasterSize, cudaMemcpyHostToDevice, t->st));
-		TCK(launch_pack_weights(t->master, t->wt, t->st));
+		TCK(pack_trainer(t));
 		TCK(cudaStreamSynchronize(t->st));
 	} else {
 		TCK(cudaMemcpyAsync(master.data(), t->master, sizeof(float) * kMlpMasterSize, cudaMemcpyDeviceToHost, t->st));
@@ -599,7 +831,7 @@ bm4dof_status bm4dof_trainer_grad(bm4dof_trainer *t, const float *feat, const fl
 	clear_error();
 	if (!trainer_ok(t, feat, target, n)) return BM4DOF_ERR_ARGUMENT;
 	TCK(cudaSetDevice(t->device));
-	bm4dof_status s = forward_backward(t, feat, target, n);
+	bm4dof_status s = train_batch(t, feat, target, n, Update{});
 	if (s != BM4DOF_OK) return s;
 	std::vector<float> g(kMlpMasterSize);
 	float l = 0.f;
@@ -617,15 +849,18 @@ bm4dof_status bm4dof_trainer_step(bm4dof_trainer *t, const float *feat, const fl
 	clear_error();
 	if (!trainer_ok(t, feat, target, n)) return BM4DOF_ERR_ARGUMENT;
 	TCK(cudaSetDevice(t->device));
-	bm4dof_status s = forward_backward(t, feat, target, n);
+	Update u{};
+	u.step = 1;
+	u.lr = lr;
+	u.b1 = 0.9f;
+	u.b2 = 0.999f;
+	u.eps = 1e-8f;
+	u.wd = weight_decay;
+	u.c1 = 1.f - std::pow(u.b1, (float)(t->step + 1));
+	u.c2 = 1.f - std::pow(u.b2, (float)(t->step + 1));
+	bm4dof_status s = train_batch(t, feat, target, n, u);
 	if (s != BM4DOF_OK) return s;
 	t->step++;
-	const float b1 = 0.9f, b2 = 0.999f;
-	const float c1 = 1.f - std::pow(b1, (float)t->step), c2 = 1.f - std::pow(b2, (float)t->step);
-	adamw_kernel<<<blocks_for(kMlpMasterSize, 256), 256, 0, t->st>>>(t->master, t->grad, t->m1, t->m2,
-	                                                                   kMlpMasterSize, lr, b1, b2, 1e-8f,
-	                                                                   weight_decay, c1, c2);
-	TCK(launch_pack_weights(t->master, t->wt, t->st));
 	if (loss) {
 		float l = 0.f;
 		TCK(cudaMemcpyAsync(&l, t->loss, sizeof(float), cudaMemcpyDeviceToHost, t->st));
