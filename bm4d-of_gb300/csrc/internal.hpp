@@ -188,7 +188,8 @@ struct Tvl1Params {
 };
 int tvl1_scales(int nx, int ny, int nscales, float zfactor);
 size_t tvl1_workspace_floats(int nx, int ny, int npairs, int nscales, float zfactor);
-cudaError_t tvl1_flow(const float *I0, const float *I1, int nx, int ny, int npairs, const Tvl1Params &p, float *u,
-                      float *v, float *ws, int *iws, int nsm, cudaStream_t st, std::string &why);
+cudaError_t tvl1_flow(const float *I0, const float *I1, int nx, int ny, int npairs, bool mirrored,
+                      const Tvl1Params &p, float *u, float *v, float *ws, int *iws, int nsm, cudaStream_t st,
+                      std::string &why);
 
 }  // namespace bm4dof

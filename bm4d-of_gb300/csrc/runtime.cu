@@ -1798,15 +1798,24 @@ bm4dof_status tvl1_setup(const bm4dof_tvl1_params *in, unsigned W, unsigned H, T
 	return BM4DOF_OK;
 }
 
+bm4dof_status tvl1_timed_out()
+{
+	set_error("bm4dof_tvl1: a barrier of the fixed-point iterations ran into its limit");
+	return BM4DOF_ERR_CUDA;
+}
+
+// n pairs; mirrored: the second half of them is the first backwards, and dI0
+// and dI1 hold n / 2 images
 bm4dof_status tvl1_run(bm4dof_ctx *ctx, const float *dI0, const float *dI1, unsigned W, unsigned H, unsigned n,
-                       const Tvl1Params &p, float *du, float *dv)
+                       bool mirrored, const Tvl1Params &p, float *du, float *dv, int *timed_out)
 {
 	float *ws;
 	int *iws;
 	DBUF("tvl1_ws", tvl1_workspace_floats((int)W, (int)H, (int)n, p.nscales, p.zfactor), ws);
 	DBUF("tvl1_iws", 2 * (size_t)n + 2, iws);
 	std::string why;
-	cudaError_t e = tvl1_flow(dI0, dI1, (int)W, (int)H, (int)n, p, du, dv, ws, iws, ctx->nsm, ctx->st, why);
+	cudaError_t e = tvl1_flow(dI0, dI1, (int)W, (int)H, (int)n, mirrored, p, du, dv, ws, iws, ctx->nsm, ctx->st, why);
+	if (e == cudaSuccess) e = cudaMemcpyAsync(timed_out, iws + 2 * n, sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
 	if (e != cudaSuccess) {
 		cudaGetLastError();
 		set_error("bm4dof_tvl1: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
@@ -1846,7 +1855,8 @@ bm4dof_status bm4dof_tvl1_pairs(bm4dof_ctx *ctx, const float *I0, const float *I
 	CK(cudaEventRecord(ctx->t_begin, ctx->st));
 	CK(cudaMemcpyAsync(d0, I0, sizeof(float) * plane * n, cudaMemcpyDefault, ctx->st));
 	CK(cudaMemcpyAsync(d1, I1, sizeof(float) * plane * n, cudaMemcpyDefault, ctx->st));
-	bm4dof_status s = tvl1_run(ctx, d0, d1, W, H, n, p, du, dv);
+	int timed_out = 0;
+	bm4dof_status s = tvl1_run(ctx, d0, d1, W, H, n, false, p, du, dv, &timed_out);
 	if (s != BM4DOF_OK) return s;
 	// [pair][2][y][x]
 	CK(cudaMemcpy2DAsync(duv, sizeof(float) * plane * 2, du, sizeof(float) * plane, sizeof(float) * plane, n,
@@ -1856,6 +1866,7 @@ bm4dof_status bm4dof_tvl1_pairs(bm4dof_ctx *ctx, const float *I0, const float *I
 	CK(cudaMemcpyAsync(uv, duv, sizeof(float) * plane * 2 * n, cudaMemcpyDefault, ctx->st));
 	CK(cudaEventRecord(ctx->t_end, ctx->st));
 	CK(cudaStreamSynchronize(ctx->st));
+	if (timed_out) return tvl1_timed_out();
 	for (int k = 0; k < 5; k++) ctx->ms[k] = 0.f;
 	cudaEventElapsedTime(&ctx->ms[4], ctx->t_begin, ctx->t_end);
 	return BM4DOF_OK;
@@ -1876,10 +1887,8 @@ bm4dof_status bm4dof_tvl1_video(bm4dof_ctx *ctx, const float *video, unsigned W,
 	tvl1_setup(params, W, H, p);
 	const size_t plane = (size_t)W * H;
 	const unsigned n = 2 * (F - 1);
-	float *dvid, *d0, *d1, *du, *dv, *dff, *dbf;
+	float *dvid, *du, *dv, *dff, *dbf;
 	DBUF("tvl1_video", plane * F, dvid);
-	DBUF("tvl1_i0", plane * n, d0);
-	DBUF("tvl1_i1", plane * n, d1);
 	DBUF("tvl1_u", plane * n, du);
 	DBUF("tvl1_v", plane * n, dv);
 	DBUF("tvl1_ff", plane * 2 * F, dff);
@@ -1892,12 +1901,8 @@ bm4dof_status bm4dof_tvl1_video(bm4dof_ctx *ctx, const float *video, unsigned W,
 	CK(cudaEventRecord(ctx->t_begin, st));
 	CK(cudaMemcpyAsync(dvid, video, sizeof(float) * plane * F, cudaMemcpyDefault, st));
 	// pairs 0..F-2: t -> t+1 (forward); F-1..2F-3: t+1 -> t (backward of t+1)
-	const size_t fb = sizeof(float) * plane * (F - 1);
-	CK(cudaMemcpyAsync(d0, dvid, fb, cudaMemcpyDeviceToDevice, st));
-	CK(cudaMemcpyAsync(d1, dvid + plane, fb, cudaMemcpyDeviceToDevice, st));
-	CK(cudaMemcpyAsync(d0 + plane * (F - 1), dvid + plane, fb, cudaMemcpyDeviceToDevice, st));
-	CK(cudaMemcpyAsync(d1 + plane * (F - 1), dvid, fb, cudaMemcpyDeviceToDevice, st));
-	bm4dof_status s = tvl1_run(ctx, d0, d1, W, H, n, p, du, dv);
+	int timed_out = 0;
+	bm4dof_status s = tvl1_run(ctx, dvid, dvid + plane, W, H, n, true, p, du, dv, &timed_out);
 	if (s != BM4DOF_OK) return s;
 	const size_t pb = sizeof(float) * plane;
 	// fflow[t] = pair t (t < F-1), fflow[F-1] = fflow[F-2];
@@ -1912,6 +1917,7 @@ bm4dof_status bm4dof_tvl1_video(bm4dof_ctx *ctx, const float *video, unsigned W,
 	CK(cudaMemcpyAsync(bflow, dbf, 2 * pb * F, cudaMemcpyDefault, st));
 	CK(cudaEventRecord(ctx->t_end, st));
 	CK(cudaStreamSynchronize(st));
+	if (timed_out) return tvl1_timed_out();
 	for (int k = 0; k < 5; k++) ctx->ms[k] = 0.f;
 	cudaEventElapsedTime(&ctx->ms[4], ctx->t_begin, ctx->t_end);
 	return BM4DOF_OK;
