@@ -145,9 +145,9 @@ constexpr int kMlpOffW1 = 0, kMlpOffB1 = kMlpInPad * kMlpHid, kMlpOffW2 = kMlpOf
               kMlpOffB2 = kMlpOffW2 + kMlpHid * kMlpHid, kMlpOffW3 = kMlpOffB2 + kMlpHid,
               kMlpOffB3 = kMlpOffW3 + kMlpHid * kMlpOutN, kMlpMasterSize = kMlpOffB3 + kMlpOutN;
 constexpr int kMlpPublicSize = kMlpMasterSize - (kMlpInPad - kMlpIn) * kMlpHid;
-constexpr int kMlpWtSize = kMlpHid * kMlpInPad + kMlpHid * kMlpHid + kMlpOutN * kMlpHid;
+constexpr int kMlpWtSize = kMlpHid * 96 + kMlpHid * kMlpHid + kMlpOutN * kMlpHid;   // inputs padded to 96
 struct MlpWeights {
-	const __nv_bfloat16 *wt1, *wt2, *wt3;   // transposed [out][in]
+	const __nv_bfloat16 *frag;   // in MMA fragment order (mlp.cu)
 	const float *b1, *b2, *b3;
 };
 MlpWeights mlp_weights(const uint16_t *wt, const float *master);

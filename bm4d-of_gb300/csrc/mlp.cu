@@ -10,9 +10,8 @@
 //     b2[256] W3[256][64] b3[64]  -- W[in][out]
 //   device master (float): the same with W1 padded to [80][256] (rows 65..79
 //     stay zero: their inputs are zero, so their gradients are zero)
-//   device working copy (bf16): Wt1[256][80] Wt2[256][256] Wt3[64][256] --
-//     transposed so that the two k-adjacent elements of an MMA B fragment are
-//     one 32-bit load
+//   device working copy (bf16): the matrices in the order of the MMA's B
+//     fragments, 16 bytes a lane (frag_at)
 //   features: bf16 [rows][80] (65 used), gains: float [rows][64]
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,8 +33,6 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 constexpr int kIn = 65, kInP = 80, kHid = 256, kOut = 64;
-constexpr int kRowsPerCta = 64;          // 4 warps x 16 rows
-constexpr int kActStride = kHid + 8;     // bf16 row pitch: conflict-free fragment loads
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
@@ -59,89 +56,14 @@ __device__ __forceinline__ float gelu_grad(float x)
 	return cdf + x * pdf;
 }
 
-__device__ __forceinline__ uint32_t ld_u32(const bf16 *p) { return *reinterpret_cast<const uint32_t *>(p); }
-
-// One dense layer for the 16 rows [wr, wr+16) of a warp: out = act(in . W + b)
-// with in a bf16 shared tile of K columns and Wt[N][K] in global memory.
-// ACT 0: GELU into the bf16 shared tile `out`; ACT 1: sigmoid into the float rows
-// of `gout`.
-template <int K, int N, int ACT>
-__device__ __forceinline__ void dense(const bf16 *in, bf16 *out, const bf16 *__restrict__ Wt,
-                                      const float *__restrict__ bias, int wr, long long row0, long long n,
-                                      float *gout)
+__device__ __forceinline__ void ldmatrix(uint32_t (&r)[4], const bf16 *p)
 {
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll 1
-	for (int nc = 0; nc < N; nc += 64) {
-		float acc[8][4];
-#pragma unroll
-		for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-#pragma unroll 4
-		for (int k0 = 0; k0 < K; k0 += 16) {
-			uint32_t a[4];
-			a[0] = ld_u32(in + (wr + g) * kActStride + k0 + 2 * t);
-			a[1] = ld_u32(in + (wr + g + 8) * kActStride + k0 + 2 * t);
-			a[2] = ld_u32(in + (wr + g) * kActStride + k0 + 8 + 2 * t);
-			a[3] = ld_u32(in + (wr + g + 8) * kActStride + k0 + 8 + 2 * t);
-#pragma unroll
-			for (int j = 0; j < 8; j++) {
-				const bf16 *wp = Wt + (size_t)(nc + j * 8 + g) * K + k0 + 2 * t;
-				mma_bf16(acc[j], a, __ldg(reinterpret_cast<const unsigned *>(wp)),
-				         __ldg(reinterpret_cast<const unsigned *>(wp + 8)));
-			}
-		}
-#pragma unroll
-		for (int j = 0; j < 8; j++) {
-			const int c = nc + j * 8 + 2 * t;
-			const float b0 = __ldg(bias + c), b1 = __ldg(bias + c + 1);
-#pragma unroll
-			for (int h = 0; h < 2; h++) {
-				const int r = wr + g + 8 * h;
-				const long long row = row0 + r;
-				const float v0 = acc[j][2 * h] + b0, v1 = acc[j][2 * h + 1] + b1;
-				if (ACT == 0) {
-					const bf16 o0 = __float2bfloat16_rn(gelu(v0)), o1 = __float2bfloat16_rn(gelu(v1));
-					out[r * kActStride + c] = o0;
-					out[r * kActStride + c + 1] = o1;
-				} else if (row < n) {
-					gout[row * N + c] = 1.f / (1.f + expf(-v0));
-					gout[row * N + c + 1] = 1.f / (1.f + expf(-v1));
-				}
-			}
-		}
-	}
+	const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+	             : "r"(s)
+	             : "memory");
 }
-
-// Forward pass over n feature rows.  Each warp owns 16 rows of the CTA's two
-// activation tiles, so the layers need only warp-level synchronisation.
-__global__ void __launch_bounds__(128)
-mlp_forward_kernel(const bf16 *__restrict__ X, long long n, MlpWeights w, float *__restrict__ out)
-{
-	extern __shared__ __align__(16) unsigned char msm[];
-	bf16 *A = reinterpret_cast<bf16 *>(msm);
-	bf16 *B = A + kRowsPerCta * kActStride;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int wr = warp * 16;
-	for (long long r0 = (long long)blockIdx.x * kRowsPerCta; r0 < n; r0 += (long long)gridDim.x * kRowsPerCta) {
-		// features of the warp's rows: 16 rows x 80 bf16 = 160 16-byte pieces
-		for (int i = lane; i < 16 * (kInP / 8); i += 32) {
-			const int rr = i / (kInP / 8), c8 = i % (kInP / 8);
-			const long long row = r0 + wr + rr;
-			uint4 v = make_uint4(0, 0, 0, 0);
-			if (row < n) v = __ldg(reinterpret_cast<const uint4 *>(X + row * kInP) + c8);
-			*reinterpret_cast<uint4 *>(B + (wr + rr) * kActStride + c8 * 8) = v;
-		}
-		__syncwarp();
-		dense<kInP, kHid, 0>(B, A, w.wt1, w.b1, wr, r0, n, nullptr);
-		__syncwarp();
-		dense<kHid, kHid, 0>(A, B, w.wt2, w.b2, wr, r0, n, nullptr);
-		__syncwarp();
-		dense<kHid, kOut, 1>(B, nullptr, w.wt3, w.b3, wr, r0, n, out);
-		__syncwarp();
-	}
-}
-
-constexpr size_t kForwardSmem = sizeof(bf16) * 2 * kRowsPerCta * kActStride;
 
 // float features [n][65] -> bf16 [n][80] (zero padded)
 __global__ void pack_features_kernel(const float *__restrict__ f, long long n, bf16 *__restrict__ X)
@@ -153,6 +75,124 @@ __global__ void pack_features_kernel(const float *__restrict__ f, long long n, b
 		X[i] = __float2bfloat16_rn(c < kIn ? f[r * kIn + c] : 0.f);
 	}
 }
+
+// ---------------------------------------------------------------------------
+// Weights as B operands of mma.m16n8k16, in fragment order: for a tile of 8
+// outputs and a pair of k-steps, lane (g = lane / 4, t = lane % 4) holds
+// k = 2t, 2t+1, 2t+8, 2t+9 of output g of both steps in 16 bytes.
+// ---------------------------------------------------------------------------
+constexpr int kInF = 96;                 // inputs padded to whole pairs of k-steps
+constexpr int kFragF1 = 0, kFragF2 = kFragF1 + kInF * kHid, kFragF3 = kFragF2 + kHid * kHid,
+              kFragB3 = kFragF3 + kHid * kOut, kFragB2 = kFragB3 + kOut * kHid, kFragSize = kFragB2 + kHid * kHid;
+static_assert(kFragB3 == kMlpWtSize, "the forward operands");
+
+// Place of B(k, n) in a fragment-ordered operand of K rows.
+__host__ __device__ __forceinline__ int frag_at(int k, int n, int K)
+{
+	const int pair = k >> 5, ks = k >> 4 & 1, kk = k & 15;
+	const int t = (kk & 7) >> 1, half = kk >> 3, lane = (n & 7) * 4 + t;
+	return (((n >> 3) * (K >> 5) + pair) * 32 + lane) * 8 + ks * 4 + half * 2 + (kk & 1);
+}
+
+// acc[mi][j] = A (MI x 16 rows, K columns, shared, pitch ldA, 16-byte rows) . B tiles tile0 + j
+template <int K, int MI, int NT>
+__device__ __forceinline__ void rows_mma(const bf16 *A, int ldA, const bf16 *__restrict__ B, int tile0,
+                                         float (&acc)[MI][NT][4])
+{
+	const int lane = threadIdx.x & 31;
+	const bf16 *ap = A + ((lane & 7) + (lane & 8)) * ldA + (lane >> 4) * 8;
+#pragma unroll
+	for (int mi = 0; mi < MI; mi++)
+#pragma unroll
+		for (int j = 0; j < NT; j++) acc[mi][j][0] = acc[mi][j][1] = acc[mi][j][2] = acc[mi][j][3] = 0.f;
+#pragma unroll 4
+	for (int p = 0; p < K / 32; p++) {
+		uint4 b[NT];
+#pragma unroll
+		for (int j = 0; j < NT; j++)
+			b[j] = __ldg(reinterpret_cast<const uint4 *>(B) + ((size_t)(tile0 + j) * (K / 32) + p) * 32 + lane);
+#pragma unroll
+		for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+			for (int mi = 0; mi < MI; mi++) {
+				uint32_t a[4];
+				ldmatrix(a, ap + mi * 16 * ldA + p * 32 + ks * 16);
+#pragma unroll
+				for (int j = 0; j < NT; j++) mma_bf16(acc[mi][j], a, ks ? b[j].z : b[j].x, ks ? b[j].w : b[j].y);
+			}
+	}
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b)
+{
+	__nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+	return *reinterpret_cast<uint32_t *>(&v);
+}
+
+// Forward pass over n feature rows, 64 rows a CTA.  A warp takes 32 (the last
+// layer: 8) columns of all 64 rows, so that a fragment of the weights, 16 bytes
+// a lane out of L2, serves eight products; the activations come from shared
+// memory by ldmatrix.
+//
+// What bounds it: the tensor cores' rate through mma.sync and erff.  1.36 million
+// rows: 5.1 -> 1.45 ms (16 rows a warp, two 4-byte loads of weights a product
+// before).
+constexpr int kFwdRows = 64, kFwdThreads = 256;
+
+__global__ void __launch_bounds__(kFwdThreads, 2)
+mlp_forward_kernel(const bf16 *__restrict__ X, long long n, MlpWeights w, float *__restrict__ out)
+{
+	constexpr int P = kHid + 8;          // row pitch without bank conflicts
+	extern __shared__ __align__(16) unsigned char msm[];
+	bf16 *A = reinterpret_cast<bf16 *>(msm), *B = A + kFwdRows * P;
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+	auto hidden = [&](float (&p)[4][4][4], const float *bias, bf16 *to) {
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const int c = warp * 32 + j * 8 + 2 * t;
+			const float b0 = __ldg(bias + c), b1 = __ldg(bias + c + 1);
+#pragma unroll
+			for (int mi = 0; mi < 4; mi++)
+#pragma unroll
+				for (int h = 0; h < 2; h++)
+					*reinterpret_cast<uint32_t *>(to + (mi * 16 + g + 8 * h) * P + c) =
+					    pack_bf16(gelu(p[mi][j][2 * h] + b0), gelu(p[mi][j][2 * h + 1] + b1));
+		}
+	};
+	for (long long r0 = (long long)blockIdx.x * kFwdRows; r0 < n; r0 += (long long)gridDim.x * kFwdRows) {
+		// 64 rows of 96 bf16 (80 in memory, then zeros) in 16-byte pieces
+		for (int i = tid; i < kFwdRows * (kInF / 8); i += kFwdThreads) {
+			const int r = i / (kInF / 8), c8 = i % (kInF / 8);
+			uint4 v = make_uint4(0, 0, 0, 0);
+			if (r0 + r < n && c8 < kInP / 8) v = __ldg(reinterpret_cast<const uint4 *>(X + (r0 + r) * kInP) + c8);
+			*reinterpret_cast<uint4 *>(B + r * P + c8 * 8) = v;
+		}
+		__syncthreads();
+		float p[4][4][4];
+		rows_mma<kInF, 4, 4>(B, P, w.frag + kFragF1, warp * 4, p);
+		hidden(p, w.b1, A);
+		__syncthreads();
+		rows_mma<kHid, 4, 4>(A, P, w.frag + kFragF2, warp * 4, p);
+		hidden(p, w.b2, B);
+		__syncthreads();
+		float o[4][1][4];
+		rows_mma<kHid, 4, 1>(B, P, w.frag + kFragF3, warp, o);
+		const int c = warp * 8 + 2 * t;
+		const float b0 = __ldg(w.b3 + c), b1 = __ldg(w.b3 + c + 1);
+#pragma unroll
+		for (int mi = 0; mi < 4; mi++)
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				const long long row = r0 + mi * 16 + g + 8 * h;
+				if (row < n)
+					*reinterpret_cast<float2 *>(out + row * kOut + c) =
+					    make_float2(1.f / (1.f + expf(-(o[mi][0][2 * h] + b0))), 1.f / (1.f + expf(-(o[mi][0][2 * h + 1] + b1))));
+			}
+		__syncthreads();
+	}
+}
+
+constexpr size_t kForwardSmem = sizeof(bf16) * 2 * kFwdRows * (kHid + 8);
 
 // ---------------------------------------------------------------------------
 // Training.  One step is three launches:
@@ -170,58 +210,10 @@ __global__ void pack_features_kernel(const float *__restrict__ f, long long n, b
 // of one wave of CTAs (4.8 GFLOP are 3 us of the tensor cores' time), the
 // weights' trip through L2 to every CTA, and erff.
 //
-// Weights as B operands of mma.m16n8k16, in fragment order: for a tile of 8
-// outputs and a pair of k-steps, lane (g = lane / 4, t = lane % 4) holds
-// k = 2t, 2t+1, 2t+8, 2t+9 of output g of both steps in 16 bytes.
 // ---------------------------------------------------------------------------
 constexpr int kTrainRows = 32, kTrainThreads = 512;   // rows and threads per CTA of train_rows_kernel
 constexpr int kGradTile = 64, kMaxSplits = 16, kSplitRows = 512;
-constexpr int kInF = 96;                 // inputs padded to whole pairs of k-steps
-constexpr int kFragF1 = 0, kFragF2 = kFragF1 + kInF * kHid, kFragF3 = kFragF2 + kHid * kHid,
-              kFragB3 = kFragF3 + kHid * kOut, kFragB2 = kFragB3 + kOut * kHid, kFragSize = kFragB2 + kHid * kHid;
 constexpr int kBiases = kHid + kHid + kOut;
-
-// Place of B(k, n) in a fragment-ordered operand of K rows.
-__host__ __device__ __forceinline__ int frag_at(int k, int n, int K)
-{
-	const int pair = k >> 5, ks = k >> 4 & 1, kk = k & 15;
-	const int t = (kk & 7) >> 1, half = kk >> 3, lane = (n & 7) * 4 + t;
-	return (((n >> 3) * (K >> 5) + pair) * 32 + lane) * 8 + ks * 4 + half * 2 + (kk & 1);
-}
-
-// acc[mi][j] = A (MI x 16 rows, K columns, shared, pitch ldA) . B tiles tile0 + j
-template <int K, int MI, int NT>
-__device__ __forceinline__ void rows_mma(const bf16 *A, int ldA, const bf16 *__restrict__ B, int tile0,
-                                         float (&acc)[MI][NT][4])
-{
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-	for (int mi = 0; mi < MI; mi++)
-#pragma unroll
-		for (int j = 0; j < NT; j++) acc[mi][j][0] = acc[mi][j][1] = acc[mi][j][2] = acc[mi][j][3] = 0.f;
-#pragma unroll 4
-	for (int p = 0; p < K / 32; p++) {
-		uint4 b[NT];
-#pragma unroll
-		for (int j = 0; j < NT; j++)
-			b[j] = __ldg(reinterpret_cast<const uint4 *>(B) + ((size_t)(tile0 + j) * (K / 32) + p) * 32 + lane);
-#pragma unroll
-		for (int ks = 0; ks < 2; ks++)
-#pragma unroll
-			for (int mi = 0; mi < MI; mi++) {
-				const bf16 *r = A + (mi * 16 + g) * ldA + p * 32 + ks * 16 + 2 * t;
-				const uint32_t a[4] = {ld_u32(r), ld_u32(r + 8 * ldA), ld_u32(r + 8), ld_u32(r + 8 * ldA + 8)};
-#pragma unroll
-				for (int j = 0; j < NT; j++) mma_bf16(acc[mi][j], a, ks ? b[j].z : b[j].x, ks ? b[j].w : b[j].y);
-			}
-	}
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b)
-{
-	__nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-	return *reinterpret_cast<uint32_t *>(&v);
-}
 
 // Sum of a column's values over the lanes that hold its rows (g = 0 .. 7).
 __device__ __forceinline__ float column_sum(float v)
@@ -444,36 +436,29 @@ weight_grad_kernel(const bf16 *__restrict__ X, const bf16 *__restrict__ H1, cons
 		}
 }
 
-// The weight's BF16 copies: the transposed one of the inference kernel and the
-// fragment-ordered ones (frag may be null).
-__device__ __forceinline__ void store_weight(int i, float v, bf16 *wt, bf16 *frag)
+// The weight's BF16 copies: in the forward pass' operand and, for training, in the
+// backward one's.
+__device__ __forceinline__ void store_weight(int i, float v, bf16 *frag, bool train)
 {
 	const bf16 b = __float2bfloat16_rn(v);
 	if (i < kMlpOffB1) {
-		const int k = i / kHid, o = i % kHid;
-		wt[o * kInP + k] = b;
-		if (frag) frag[kFragF1 + frag_at(k, o, kInF)] = b;
+		frag[kFragF1 + frag_at(i / kHid, i % kHid, kInF)] = b;
 	} else if (i >= kMlpOffW2 && i < kMlpOffB2) {
 		const int j = i - kMlpOffW2, k = j / kHid, o = j % kHid;
-		wt[kHid * kInP + o * kHid + k] = b;
-		if (frag) {
-			frag[kFragF2 + frag_at(k, o, kHid)] = b;
-			frag[kFragB2 + frag_at(o, k, kHid)] = b;
-		}
+		frag[kFragF2 + frag_at(k, o, kHid)] = b;
+		if (train) frag[kFragB2 + frag_at(o, k, kHid)] = b;
 	} else if (i >= kMlpOffW3 && i < kMlpOffB3) {
 		const int j = i - kMlpOffW3, k = j / kOut, o = j % kOut;
-		wt[kHid * kInP + kHid * kHid + o * kHid + k] = b;
-		if (frag) {
-			frag[kFragF3 + frag_at(k, o, kHid)] = b;
-			frag[kFragB3 + frag_at(o, k, kOut)] = b;
-		}
+		frag[kFragF3 + frag_at(k, o, kHid)] = b;
+		if (train) frag[kFragB3 + frag_at(o, k, kOut)] = b;
 	}
 }
 
-__global__ void pack_weights_kernel(const float *__restrict__ m, bf16 *__restrict__ wt, bf16 *__restrict__ frag)
+// (the inputs past the master's 80 are cleared by the caller)
+__global__ void pack_weights_kernel(const float *__restrict__ m, bf16 *__restrict__ frag, int train)
 {
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpMasterSize; i += gridDim.x * blockDim.x)
-		store_weight(i, m[i], wt, frag);
+		store_weight(i, m[i], frag, train != 0);
 }
 
 __device__ __forceinline__ bool is_bias(int i)
@@ -488,7 +473,7 @@ struct Update {
 	int step;
 	float *p, *m, *v;
 	float lr, b1, b2, eps, wd, c1, c2;
-	bf16 *wt, *frag;
+	bf16 *frag;
 };
 
 // Sums of the splits (weights: a thread each; biases and the loss: a warp each),
@@ -510,7 +495,7 @@ update_kernel(Update u)
 		if (!bias) q -= u.lr * u.wd * q;
 		q -= u.lr * (mi / u.c1) / (sqrtf(vi / u.c2) + u.eps);
 		u.p[i] = q;
-		if (!bias) store_weight(i, q, u.wt, u.frag);
+		if (!bias) store_weight(i, q, u.frag, true);
 	};
 	const int nthreads = gridDim.x * blockDim.x, id = blockIdx.x * blockDim.x + threadIdx.x;
 	for (int i = id; i < kMlpMasterSize; i += nthreads) {
@@ -547,25 +532,24 @@ cudaError_t launch_mlp_forward(const uint16_t *X, long long n, const MlpWeights 
 	cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                     (int)kForwardSmem);
 	if (e != cudaSuccess) return e;
-	const long long need = (n + kRowsPerCta - 1) / kRowsPerCta;
-	const int nb = (int)std::min<long long>(need, (long long)nsm * 3);
-	mlp_forward_kernel<<<nb, 128, kForwardSmem, st>>>(reinterpret_cast<const bf16 *>(X), n, w, out);
+	const long long need = (n + kFwdRows - 1) / kFwdRows;
+	const int nb = (int)std::min<long long>(need, (long long)nsm * 2);
+	mlp_forward_kernel<<<nb, kFwdThreads, kForwardSmem, st>>>(reinterpret_cast<const bf16 *>(X), n, w, out);
 	return cudaGetLastError();
 }
 
 cudaError_t launch_pack_weights(const float *master, uint16_t *wt, cudaStream_t st)
 {
-	pack_weights_kernel<<<256, 256, 0, st>>>(master, reinterpret_cast<bf16 *>(wt), nullptr);
+	cudaError_t e = cudaMemsetAsync(wt, 0, sizeof(bf16) * kFragF2, st);
+	if (e != cudaSuccess) return e;
+	pack_weights_kernel<<<256, 256, 0, st>>>(master, reinterpret_cast<bf16 *>(wt), 0);
 	return cudaGetLastError();
 }
 
 MlpWeights mlp_weights(const uint16_t *wt, const float *master)
 {
 	MlpWeights w;
-	const bf16 *b = reinterpret_cast<const bf16 *>(wt);
-	w.wt1 = b;
-	w.wt2 = b + kHid * kInP;
-	w.wt3 = b + kHid * kInP + kHid * kHid;
+	w.frag = reinterpret_cast<const bf16 *>(wt);
 	w.b1 = master + kMlpOffB1;
 	w.b2 = master + kMlpOffB2;
 	w.b3 = master + kMlpOffB3;
@@ -600,7 +584,6 @@ struct bm4dof_trainer {
 	long long step = 0;
 	cudaStream_t st = nullptr;
 	float *master = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
-	uint16_t *wt = nullptr;
 	bf16 *frag = nullptr;        // the weights in fragment order
 	// activations and gradients of one batch (rows padded to whole CTAs)
 	bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *D1 = nullptr, *D2 = nullptr, *D3 = nullptr;
@@ -620,7 +603,7 @@ namespace {
 
 void free_trainer(bm4dof_trainer *t)
 {
-	void *ps[] = {t->master, t->grad, t->m1, t->m2, t->wt, t->frag, t->X, t->H1, t->H2, t->D1, t->D2, t->D3,
+	void *ps[] = {t->master, t->grad, t->m1, t->m2, t->frag, t->X, t->H1, t->H2, t->D1, t->D2, t->D3,
 	              t->part, t->bias_part, t->loss_part, t->loss};
 	for (void *p : ps)
 		if (p) cudaFree(p);
@@ -663,7 +646,6 @@ bm4dof_status train_batch(bm4dof_trainer *t, const float *feat, const float *tar
 	u.p = t->master;
 	u.m = t->m1;
 	u.v = t->m2;
-	u.wt = reinterpret_cast<bf16 *>(t->wt);
 	u.frag = t->frag;
 	update_kernel<<<blocks_for(kMlpMasterSize, 256), 256, 0, st>>>(u);
 	TCK(cudaGetLastError());
@@ -672,7 +654,7 @@ bm4dof_status train_batch(bm4dof_trainer *t, const float *feat, const float *tar
 
 cudaError_t pack_trainer(bm4dof_trainer *t)
 {
-	pack_weights_kernel<<<256, 256, 0, t->st>>>(t->master, reinterpret_cast<bf16 *>(t->wt), t->frag);
+	pack_weights_kernel<<<256, 256, 0, t->st>>>(t->master, t->frag, 1);
 	return cudaGetLastError();
 }
 
@@ -712,7 +694,6 @@ bm4dof_status bm4dof_trainer_create(bm4dof_trainer **out, int device, unsigned b
 	          cudaMalloc(&t->grad, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->m1, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
 	          cudaMalloc(&t->m2, sizeof(float) * kMlpMasterSize) == cudaSuccess &&
-	          cudaMalloc(&t->wt, sizeof(uint16_t) * kMlpWtSize) == cudaSuccess &&
 	          cudaMalloc(&t->frag, sizeof(bf16) * kFragSize) == cudaSuccess &&
 	          cudaMalloc(&t->X, sizeof(bf16) * B * kInF) == cudaSuccess &&
 	          cudaMalloc(&t->H1, sizeof(bf16) * B * kHid) == cudaSuccess &&
@@ -879,7 +860,7 @@ bm4dof_status bm4dof_trainer_predict(bm4dof_trainer *t, const float *feat, unsig
 	}
 	TCK(cudaSetDevice(t->device));
 	pack_features_kernel<<<blocks_for((long long)n * kInP, 256), 256, 0, t->st>>>(feat, n, t->X);
-	TCK(launch_mlp_forward(reinterpret_cast<const uint16_t *>(t->X), n, mlp_weights(t->wt, t->master), gains,
+	TCK(launch_mlp_forward(reinterpret_cast<const uint16_t *>(t->X), n, mlp_weights(reinterpret_cast<const uint16_t *>(t->frag), t->master), gains,
 	                       t->nsm, t->st));
 	TCK(cudaStreamSynchronize(t->st));
 	return BM4DOF_OK;
