@@ -24,10 +24,10 @@
 // nSimilarPatchesPred 5x5 windows elsewhere), so the warp walks the frames
 // while the other warps of the SM hide its latency.  Frame pt's window is
 // computed in column strips (each row of the image loaded once for kR
-// vertically adjacent candidates); the predicted windows one candidate per
-// lane.  Selections, when the nearest are distinct: repeated warp minima
-// (few nearest) or a warp bitonic sort (more nearest, up to 64 candidates);
-// else an exact replay of libstdc++'s heap selection by one lane.
+// vertically adjacent candidates), a small one, like the predicted windows, two
+// candidates per lane.  Selections, when the nearest are distinct: repeated
+// warp minima (few nearest) or a warp bitonic sort (more nearest, up to 64
+// candidates); else an exact replay of libstdc++'s heap selection by one lane.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdlib>
@@ -125,6 +125,9 @@ __device__ __forceinline__ void warp_sort32(float &d0, int &i0)
 		}
 }
 
+// Candidates of frame pt up to which a lane takes two rather than a strip of kR: a
+// 7x7 window is 14 strips for 32 lanes, or one round of pairs.
+constexpr int kPairsUpTo = 128;
 constexpr int kRoundsMaxK = 5;   // repeated minima up to this K, else a bitonic sort
 
 // The K nearest of d[0..n) (1 <= K <= min(n, kMaxNp)) in the order
@@ -298,6 +301,52 @@ __device__ __forceinline__ void patch_distance2(const float *p0, const float *p1
 	}
 }
 
+// The same for reps > 1: the terms of the later passes are those of the first,
+// kept in registers, so a later pass is the additions alone.  (A call: one copy
+// of its 700 instructions for the places that need it.)
+template <int PX, int PT>
+__device__ __noinline__ float2 patch_distance2_reps(const float *p0, const float *p1, size_t rpitch, size_t tpitch,
+                                                    const float *ref, int reps)
+{
+	constexpr int N = PX * PX * PT;
+	float m0[N], m1[N], a0 = 0.f, a1 = 0.f;
+#pragma unroll
+	for (int tt = 0; tt < PT; tt++)
+#pragma unroll
+		for (int yy = 0; yy < PX; yy++) {
+			const size_t off = tt * tpitch + yy * rpitch;
+#pragma unroll
+			for (int xx = 0; xx < PX; xx++) {
+				const int k = (tt * PX + yy) * PX + xx;
+				const float rv = ref[k];
+				sqdiff2(rv, rv, __ldg(p0 + off + xx), __ldg(p1 + off + xx), m0[k], m1[k]);
+				a0 = __fadd_rn(a0, m0[k]);
+				a1 = __fadd_rn(a1, m1[k]);
+			}
+		}
+#pragma unroll 1
+	for (int r = 1; r < reps; r++)
+#pragma unroll
+		for (int k = 0; k < N; k++) {
+			a0 = __fadd_rn(a0, m0[k]);
+			a1 = __fadd_rn(a1, m1[k]);
+		}
+	return make_float2(a0, a1);
+}
+
+template <int PX, int PT, bool REPS>
+__device__ __forceinline__ float2 pair_distance(const float *p0, const float *p1, size_t rpitch, size_t tpitch,
+                                                const float *ref, int reps, int px, int pt)
+{
+	if constexpr (REPS) {
+		return patch_distance2_reps<PX, PT>(p0, p1, rpitch, tpitch, ref, reps);
+	} else {
+		float a0, a1;
+		patch_distance2<PX, PT>(p0, p1, rpitch, tpitch, ref, reps, px, pt, a0, a1);
+		return make_float2(a0, a1);
+	}
+}
+
 // Window of one centre, shifted (not clipped) into the frame
 // (nldct.cpp:1017-1027): [x0, x0 + nx) x [y0, y0 + ny).
 __device__ __forceinline__ void window_box(int cx, int cy, int sw, int tw, int th, int px, int &x0, int &y0,
@@ -333,7 +382,7 @@ __device__ __forceinline__ void predicted_window(const Image &ffl, const Image &
 	window_box(cx, cy, sp.wxp, T.w, T.h, sp.px, x0, y0, nx, ny);
 }
 
-template <int PX, int PT, int MINB>
+template <int PX, int PT, int MINB, bool REPS>
 __global__ void __launch_bounds__(32 * kWarps, MINB)
 search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 {
@@ -383,6 +432,21 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 				ncand = fnx * fny;
 				const int nit = fnx * ((fny + kR - 1) / kR);
 				nan = false;
+				if (REPS || ncand <= kPairsUpTo) {
+					for (int c = lane; c < ncand; c += 64) {
+						const int c1 = c + 32 < ncand ? c + 32 : c;
+						const int y0 = c / fnx, y1 = c1 / fnx, qx0 = fx0 + c - y0 * fnx, qx1 = fx0 + c1 - y1 * fnx,
+						          qy0 = fy0 + y0, qy1 = fy0 + y1;
+						float2 d = pair_distance<PX, PT, REPS>(src.p + src.at(T.ox + qx0, T.oy + qy0, qt, 0),
+						                                       src.p + src.at(T.ox + qx1, T.oy + qy1, qt, 0), rpitch, tpitch,
+						                                       ref, a.reps, px, sp.pt);
+						if (qx0 == x && qy0 == y) d.x = __fsub_rn(d.x, sp.dsub_bias);
+						if (qx1 == x && qy1 == y) d.y = __fsub_rn(d.y, sp.dsub_bias);
+						nan |= d.x != d.x || d.y != d.y;
+						dist[c] = d.x;
+						dist[c1] = c1 == c ? d.x : d.y;
+					}
+				} else
 				for (int it = lane; it < nit; it += 32) {
 					const int rb = it / fnx, cx = it - rb * fnx, qy0 = rb * kR;
 					float acc[kR];
@@ -433,10 +497,10 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 					const uint32_t q0 = pos[c], q1 = two ? pos[c + 32] : q0;
 					const int qx0 = (int)(q0 & 0xffffu), qy0 = (int)(q0 >> 16);
 					const int qx1 = (int)(q1 & 0xffffu), qy1 = (int)(q1 >> 16);
-					float d0, d1;
-					patch_distance2<PX, PT>(src.p + src.at(T.ox + qx0, T.oy + qy0, qt, 0),
-					                        src.p + src.at(T.ox + qx1, T.oy + qy1, qt, 0), rpitch, tpitch, ref,
-					                        a.reps, px, sp.pt, d0, d1);
+					const float2 d = pair_distance<PX, PT, REPS>(src.p + src.at(T.ox + qx0, T.oy + qy0, qt, 0),
+					                                             src.p + src.at(T.ox + qx1, T.oy + qy1, qt, 0), rpitch,
+					                                             tpitch, ref, a.reps, px, sp.pt);
+					float d0 = d.x, d1 = d.y;
 					if (qx0 == x && qy0 == y) d0 = __fsub_rn(d0, sp.dsub_bias);
 					if (qx1 == x && qy1 == y) d1 = __fsub_rn(d1, sp.dsub_bias);
 					nan |= d0 != d0;
@@ -522,10 +586,10 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 					const uint32_t q0 = pos[s0 * a.cap_pred + j0], q1 = pos[s1 * a.cap_pred + j1];
 					const int qx0 = (int)(q0 & 0xffffu), qy0 = (int)(q0 >> 16);
 					const int qx1 = (int)(q1 & 0xffffu), qy1 = (int)(q1 >> 16);
-					float d0, d1;
-					patch_distance2<PX, PT>(src.p + src.at(T.ox + qx0, T.oy + qy0, s0 ? t - k : t + k, 0),
-					                        src.p + src.at(T.ox + qx1, T.oy + qy1, s1 ? t - k : t + k, 0), rpitch,
-					                        tpitch, ref, a.reps, px, sp.pt, d0, d1);
+					const float2 d = pair_distance<PX, PT, REPS>(
+					    src.p + src.at(T.ox + qx0, T.oy + qy0, s0 ? t - k : t + k, 0),
+					    src.p + src.at(T.ox + qx1, T.oy + qy1, s1 ? t - k : t + k, 0), rpitch, tpitch, ref, a.reps, px, sp.pt);
+					float d0 = d.x, d1 = d.y;
 					if (qx0 == x && qy0 == y) d0 = __fsub_rn(d0, sp.dsub_bias);
 					if (qx1 == x && qy1 == y) d1 = __fsub_rn(d1, sp.dsub_bias);
 					dist[s0 * a.cap_pred + j0] = d0;
@@ -569,11 +633,11 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 	}
 }
 
-template <int PX, int PT, int MINB = 1>
+template <int PX, int PT, int MINB = 1, bool REPS = false>
 cudaError_t launch_t(const Image &src, const Image &ffl, const Image &bfl, const StepParams &sp, const VArgs &a,
                      int nsm, cudaStream_t st)
 {
-	auto kern = search_vbm3d_kernel<PX, PT, MINB>;
+	auto kern = search_vbm3d_kernel<PX, PT, MINB, REPS>;
 	const size_t smem = sizeof(float) * (size_t)a.per_warp * kWarps;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess) return e;
@@ -651,12 +715,20 @@ cudaError_t launch_search_vbm3d(const Image &src, const Image &ffl, const Image 
 		const char *e = std::getenv("BM4DOF_VBM3D_MINB");
 		return e ? std::atoi(e) : 8;
 	}();
+	// (repeated distances: 168 registers for the 128 terms of two candidates).
+	// 720x576x3x14 with the default parameters (8x8, 7x7 windows; reps 1, then 3):
+	// 21.3 ms with strips and every pass computed again, 14.6 now; 480x320x3x8 at
+	// sigma 20 (7x7 in step 2, without a template of its own before) 6.5 -> 3.0.
 	if (sp.px == 4 && sp.pt == 4) {
+		if (reps > 1) return launch_t<4, 4, 3, true>(src, ffl, bfl, sp, a, nsm, st);
 		if (minb == 4) return launch_t<4, 4, 4>(src, ffl, bfl, sp, a, nsm, st);
 		if (minb == 6) return launch_t<4, 4, 6>(src, ffl, bfl, sp, a, nsm, st);
 		return launch_t<4, 4, 8>(src, ffl, bfl, sp, a, nsm, st);
 	}
-	if (sp.px == 8 && sp.pt == 1) return launch_t<8, 1, 4>(src, ffl, bfl, sp, a, nsm, st);
+	if (sp.px == 8 && sp.pt == 1)
+		return reps > 1 ? launch_t<8, 1, 3, true>(src, ffl, bfl, sp, a, nsm, st) : launch_t<8, 1, 4>(src, ffl, bfl, sp, a, nsm, st);
+	if (sp.px == 7 && sp.pt == 1)
+		return reps > 1 ? launch_t<7, 1, 4, true>(src, ffl, bfl, sp, a, nsm, st) : launch_t<7, 1, 4>(src, ffl, bfl, sp, a, nsm, st);
 	return launch_t<0, 0>(src, ffl, bfl, sp, a, nsm, st);
 }
 
