@@ -72,10 +72,12 @@ cudaError_t launch_search_block(const Image &src, const Tile *tiles, int ntiles,
 
 // search_vbm3d.cu (the reference's VBM3D_SEARCH build)
 bool vbm3d_check(const StepParams &sp, const std::vector<Tile> &tiles, std::string &why);
+bool vbm3d_first_frame(const StepParams &sp, int reps, const Plan &pl, StepParams &fp);
 size_t vbm3d_smem_bytes(const StepParams &sp, int reps);
 cudaError_t launch_search_vbm3d(const Image &src, const Image &ffl, const Image &bfl, const Tile *tiles,
                                 int ntiles, const int *grid, const StepParams &sp, int reps, long long g_begin,
-                                long long g_end, uint8_t *nsimp, uint32_t *idx, int nsm, cudaStream_t st);
+                                long long g_end, uint8_t *nsimp, uint32_t *idx, int nsm, cudaStream_t st,
+                                const uint32_t *first);
 
 // search_tc.cu: tensor-core pre-screen + certified exact re-rank; the groups
 // it cannot certify are listed for launch_search (list mode)

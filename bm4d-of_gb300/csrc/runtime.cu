@@ -669,8 +669,19 @@ bm4dof_status launch_step(bm4dof_ctx *ctx, int slot, const Image &noisy, const I
 		Mark m(ctx, T_SEARCH);
 		if (sp.vbm3d) {
 			// trajectories are chained inside the search (they follow the matches)
-			CK(launch_search_vbm3d(on_noisy ? noisy : basic, ffl, bfl, S.d_tiles, ntiles, S.d_grid, sp,
-			                       on_noisy ? 1 : (int)C, 0, G, S.d_nsimp, S.d_idx, ctx->nsm, st));
+			const Image &src = on_noisy ? noisy : basic;
+			const uint32_t *first = nullptr;
+			StepParams fp;
+			if (vbm3d_first_frame(sp, on_noisy ? 1 : (int)C, pl, fp)) {
+				CK(launch_traj(ffl, bfl, S.d_tiles, ntiles, S.d_grid, fp, G, S.d_traj, st));
+				CK(cudaMemsetAsync(S.d_nsimp, 0, G, st));
+				CK(launch_search_block(src, S.d_tiles, ntiles, S.d_grid, S.d_traj, fp, pl.step, pl.nblocks, S.d_nsimp,
+				                       S.d_traj + G, nullptr, nullptr, S.d_small + 2, ctx->nsm, st));
+				first = S.d_traj + G;
+				ctx->launches += 3;
+			}
+			CK(launch_search_vbm3d(src, ffl, bfl, S.d_tiles, ntiles, S.d_grid, sp, on_noisy ? 1 : (int)C, 0, G,
+			                       S.d_nsimp, S.d_idx, ctx->nsm, st, first));
 			ctx->launches += 1;
 		} else if (S.tc_search) {
 			// tensor-core pre-screen and certified re-rank; the groups it cannot

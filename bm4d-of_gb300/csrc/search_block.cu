@@ -214,7 +214,7 @@ struct BlockArgs {
 	const unsigned *bad_source;
 	uint8_t *nsimp;
 	uint32_t *idx;
-	uint32_t *glist;                   // groups left to the per-group kernel
+	uint32_t *glist;                   // groups left to the per-group kernel (or none: nsimp stays as it is)
 	unsigned *gcount;
 	float eps;                         // relative error bound between two sums of one distance
 };
@@ -359,7 +359,7 @@ search_block_kernel(Image src, StepParams sp, BlockArgs a)
 		for (int k = 0; k < 4; k++) K[k] = min(sp.np, __reduce_add_sync(0xffffffffu, cand[k]));
 		if (__any_sync(0xffffffffu, wide) || nitems > 32 * kMaxRounds) {
 			// windows far apart (a motion boundary with a large jump)
-			if (lane < 4 && exists(lane)) a.glist[atomicAdd(a.gcount, 1u)] = (uint32_t)group(lane);
+			if (a.glist && lane < 4 && exists(lane)) a.glist[atomicAdd(a.gcount, 1u)] = (uint32_t)group(lane);
 			continue;
 		}
 		// ---- reference pixels: per row S pairs (left, right), then the middle --
@@ -595,7 +595,7 @@ search_block_kernel(Image src, StepParams sp, BlockArgs a)
 				}
 			}
 			if (!ok) {
-				if (lane == 0) a.glist[atomicAdd(a.gcount, 1u)] = (uint32_t)g;
+				if (a.glist && lane == 0) a.glist[atomicAdd(a.gcount, 1u)] = (uint32_t)g;
 				__syncwarp();
 				continue;
 			}

@@ -52,6 +52,7 @@ struct VArgs {
 	long long g_begin, g_end;
 	uint8_t *nsimp;
 	uint32_t *idx;
+	const uint32_t *first;   // [group][npf] nearest of frame pt, where nsimp is npf (or none)
 	int reps;          // passes over channel 0: 1 in step 1, C in step 2
 	int cap_win;       // most candidates of one frame (two predicted frames)
 	int cap_pred;      // most candidates of one predicted frame
@@ -430,6 +431,22 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 				int fny;
 				window_box(x, y, sp.wx, T.w, T.h, px, fx0, fy0, fnx, fny);
 				ncand = fnx * fny;
+				if (a.first && a.nsimp[g] == npf) {
+					// found by the block search, in order: their distances are formed again
+					uint32_t q = 0;
+					if (lane < npf) q = a.first[g * npf + lane];
+					const int qx = lane < npf ? (int)(q % (uint32_t)T.w) : x,
+					          qy = lane < npf ? (int)(q / (uint32_t)T.w % (uint32_t)T.h) : y;
+					const float *qp = src.p + src.at(T.ox + qx, T.oy + qy, qt, 0);
+					float2 d = pair_distance<PX, PT, REPS>(qp, qp, rpitch, tpitch, ref, a.reps, px, sp.pt);
+					if (qx == x && qy == y) d.x = __fsub_rn(d.x, sp.dsub_bias);
+					if (lane < npf) {
+						pool_d[lane] = d.x;
+						pool_i[lane] = q;
+					}
+					__syncwarp();
+					continue;
+				}
 				const int nit = fnx * ((fny + kR - 1) / kR);
 				nan = false;
 				if (REPS || ncand <= kPairsUpTo) {
@@ -680,6 +697,24 @@ bool vbm3d_check(const StepParams &sp, const std::vector<Tile> &tiles, std::stri
 	return true;
 }
 
+// Frame pt's nearest by the block search (search_block.cu) where its window is
+// larger than a warp takes in pairs, distances are summed once, and their number
+// is one that the search's power-of-two lists hold; the trajectories' buffer,
+// which the predictive search does not use, holds its positions and lists.
+// Groups that it leaves open are searched here.  854x480x12, 21x21 windows, both
+// steps: 29.8 -> 25.3 ms.
+bool vbm3d_first_frame(const StepParams &sp, int reps, const Plan &pl, StepParams &fp)
+{
+	fp = sp;
+	fp.np = sp.npf;
+	fp.wtf = fp.wtb = 0;
+	fp.tau2 = 3e38f;
+	fp.chn_search = 1;
+	const int w = 2 * ((sp.wx - 1) / 2) + 1;
+	return sp.np > 1 && reps == 1 && w * w > kPairsUpTo && (sp.npf & (sp.npf - 1)) == 0 &&
+	       1 + sp.npf <= search_frames_max(sp) && block_search_supported(fp, pl);
+}
+
 size_t vbm3d_smem_bytes(const StepParams &sp, int reps)
 {
 	const int hw = 2 * ((sp.wx - 1) / 2) + 1, hp = 2 * ((sp.wxp - 1) / 2) + 1;
@@ -690,7 +725,8 @@ size_t vbm3d_smem_bytes(const StepParams &sp, int reps)
 
 cudaError_t launch_search_vbm3d(const Image &src, const Image &ffl, const Image &bfl, const Tile *tiles,
                                 int ntiles, const int *grid, const StepParams &sp, int reps, long long g_begin,
-                                long long g_end, uint8_t *nsimp, uint32_t *idx, int nsm, cudaStream_t st)
+                                long long g_end, uint8_t *nsimp, uint32_t *idx, int nsm, cudaStream_t st,
+                                const uint32_t *first)
 {
 	if (g_end <= g_begin) return cudaSuccess;
 	if (sp.np <= 1) return launch_search(src, tiles, ntiles, grid, nullptr, sp, g_begin, g_end, nsimp, idx,
@@ -703,6 +739,7 @@ cudaError_t launch_search_vbm3d(const Image &src, const Image &ffl, const Image 
 	a.g_end = g_end;
 	a.nsimp = nsimp;
 	a.idx = idx;
+	a.first = first;
 	a.reps = reps;
 	const int hw = 2 * ((sp.wx - 1) / 2) + 1, hp = 2 * ((sp.wxp - 1) / 2) + 1;
 	a.cap_pred = sp.npf * hp * hp;
