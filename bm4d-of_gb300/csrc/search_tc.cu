@@ -18,8 +18,8 @@
 //    test the candidate against the thread's own window and keep the 32
 //    smallest a(p, q): candidates under the current 32nd smallest wait in a
 //    list of up to 32 per reference, which the warp merges into the sorted
-//    kept list with bitonic networks when it fills.  Four staging warps build the
-//    next chunk's operands while the selection warps work on the current
+//    kept list with bitonic networks, three references side by side, when one
+//    fills.  Eight staging warps build the next chunk's operands while the selection warps work on the current
 //    one (two operand buffers, two TMEM accumulators of 256 columns,
 //    mbarriers between them).  Per reference it writes the 32 candidates and
 //    a lower bound L on the exact distance of every candidate it dropped:
@@ -40,6 +40,15 @@
 //    basic estimate) keeps the order of its re-ranked 32 by default, or goes
 //    on that list too when every neighbour list must be the exact path's
 //    (BM4DOF_MIXED_CERTIFIED).
+//
+// What bounds it: the four selection warps, one per scheduler, and in them the
+// latency of their own chains (window masks, reading tensor memory, the lists)
+// rather than issue slots; the tensor cores are idle most of the time.  1.36
+// million groups (854x480x16, 13 frames of 21x21): 52.4 ms with the hits taken
+// in rounds of the whole warp, one row merged at a time and four staging warps,
+// 34.1 so; of a selection warp's cycles 19 % are merges, 16 % listing, 36 %
+// masks and keys, 22 % waits.  Two selection warps per tensor-memory quadrant
+// (16 warps) with the kept lists shared under a lock took 67 ms or more.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -58,7 +67,7 @@ constexpr int kRefs = 128;            // references per CTA (MMA M, TMEM lanes)
 constexpr int kBX = 16, kBY = 8;      // ... as a 16 x 8 block of grid positions
 constexpr int kN = 256;               // candidates per chunk (MMA N)
 constexpr int kK = 64;                // patch elements (MMA K, four k-steps of 16)
-constexpr int kThreads = 256;         // warps 0-3 select, warps 4-7 stage and issue
+constexpr int kThreads = 384;         // warps 0-3 select, warps 4-11 stage and issue
 constexpr int kTop = 32;              // approximate candidates kept per reference
 constexpr int kMaxWt = 16;            // candidate frames per reference on this path
 constexpr int kWinHalves = 16384;     // staged window capacity (FP16 values)
@@ -72,6 +81,8 @@ constexpr int kOffWin = kOffB + 2 * kN * kK * 2;          // staged window
 constexpr int kOffQn = kOffWin + kWinHalves * 2 + 64;     // 2 x 256 candidate norms
 // per reference (row of kLs words): the kept 32 (keys and candidates,
 // ascending) and up to 32 newcomers waiting for a merge
+constexpr int kMerge = 3;                                 // references merged side by side
+constexpr int kMergeFrom = 24;                            // newcomers from which a list joins a merge
 constexpr int kLs = kTop + 1;                             // row stride: rows start in distinct banks
 constexpr int kOffKd = kOffQn + 2 * kN * 4;               // kept keys: 128 x kLs
 constexpr int kOffKc = kOffKd + kRefs * kLs * 4;          // kept candidates
@@ -179,57 +190,91 @@ __device__ __forceinline__ float drop_bound(float a32, float pn, float qmax, flo
 	return d * d * 0.9999f;
 }
 
-// Warp-cooperative merge of one reference's newcomers (nd/nc, the first
-// `cnt` of its row) into its kept 32 (kd/kc, ascending): the newcomers are
+// Warp-cooperative merge of kMerge references' newcomers (the first `cnt` of
+// their rows of nd/nc) into their kept 32 (kd/kc, ascending): the newcomers are
 // sorted by a bitonic network across the lanes, the lane-wise minimum of the
 // kept list and the reversed newcomers is a bitonic sequence holding the 32
 // smallest of both, and a bitonic merge orders it.  Returns the new 32nd
-// smallest key (the threshold for newcomers) to every lane.
-__device__ __forceinline__ float merge_row(float *kd, uint32_t *kc, const float *nd, const uint32_t *nc, int row,
-                                          int cnt)
+// smallest keys (the thresholds for newcomers) to every lane.  The networks are
+// chains of 20 shuffles and selections, so several rows go side by side (a row
+// twice among them is merged twice with the same result).
+__device__ __forceinline__ void take_if_less(float &x, uint32_t &xc, float ox, uint32_t oc, bool least)
+{
+	const float a = least ? ox : x, b = least ? x : ox;
+	const bool take = a < b;
+	x = take ? ox : x;
+	xc = take ? oc : xc;
+}
+
+__device__ __forceinline__ void merge_rows(float *kd, uint32_t *kc, const float *nd, const uint32_t *nc,
+                                           const int (&row)[kMerge], const int (&cnt)[kMerge], float (&last)[kMerge])
 {
 	const int lane = threadIdx.x & 31;
-	float x = lane < cnt ? nd[row * kLs + lane] : __int_as_float(0x7f800000);
-	uint32_t xc = lane < cnt ? nc[row * kLs + lane] : 0xffffffffu;
+	float x[kMerge], y[kMerge];
+	uint32_t xc[kMerge], yc[kMerge];
+#pragma unroll
+	for (int q = 0; q < kMerge; q++) {
+		const bool on = lane < cnt[q];
+		x[q] = on ? nd[row[q] * kLs + lane] : __int_as_float(0x7f800000);
+		xc[q] = on ? nc[row[q] * kLs + lane] : 0xffffffffu;
+		y[q] = kd[row[q] * kLs + lane];
+		yc[q] = kc[row[q] * kLs + lane];
+	}
 #pragma unroll
 	for (int k = 2; k <= 32; k <<= 1)
 #pragma unroll
-		for (int j = k >> 1; j > 0; j >>= 1) {
-			const float ox = __shfl_xor_sync(0xffffffffu, x, j);
-			const uint32_t oc = __shfl_xor_sync(0xffffffffu, xc, j);
-			const bool up = (lane & k) == 0, low = (lane & j) == 0;
-			if ((low == up) ? (ox < x) : (x < ox)) { x = ox; xc = oc; }
-		}
-	float y = kd[row * kLs + lane];
-	uint32_t yc = kc[row * kLs + lane];
-	const float rx = __shfl_sync(0xffffffffu, x, 31 - lane);
-	const uint32_t rc = __shfl_sync(0xffffffffu, xc, 31 - lane);
-	if (rx < y) { y = rx; yc = rc; }
+		for (int j = k >> 1; j > 0; j >>= 1)
 #pragma unroll
-	for (int j = 16; j > 0; j >>= 1) {
-		const float oy = __shfl_xor_sync(0xffffffffu, y, j);
-		const uint32_t oc = __shfl_xor_sync(0xffffffffu, yc, j);
-		if (((lane & j) == 0) ? (oy < y) : (y < oy)) { y = oy; yc = oc; }
+			for (int q = 0; q < kMerge; q++) {
+				const float ox = __shfl_xor_sync(0xffffffffu, x[q], j);
+				const uint32_t oc = __shfl_xor_sync(0xffffffffu, xc[q], j);
+				take_if_less(x[q], xc[q], ox, oc, ((lane & k) == 0) == ((lane & j) == 0));
+			}
+#pragma unroll
+	for (int q = 0; q < kMerge; q++) {
+		const float rx = __shfl_sync(0xffffffffu, x[q], 31 - lane);
+		const uint32_t rc = __shfl_sync(0xffffffffu, xc[q], 31 - lane);
+		take_if_less(y[q], yc[q], rx, rc, true);
 	}
-	kd[row * kLs + lane] = y;
-	kc[row * kLs + lane] = yc;
-	return __shfl_sync(0xffffffffu, y, 31);
+#pragma unroll
+	for (int j = 16; j > 0; j >>= 1)
+#pragma unroll
+		for (int q = 0; q < kMerge; q++) {
+			const float oy = __shfl_xor_sync(0xffffffffu, y[q], j);
+			const uint32_t oc = __shfl_xor_sync(0xffffffffu, yc[q], j);
+			take_if_less(y[q], yc[q], oy, oc, (lane & j) == 0);
+		}
+#pragma unroll
+	for (int q = 0; q < kMerge; q++) {
+		kd[row[q] * kLs + lane] = y[q];
+		kc[row[q] * kLs + lane] = yc[q];
+		last[q] = __shfl_sync(0xffffffffu, y[q], 31);
+	}
 }
 
 // Merges every lane's newcomers whose lane is set in `need` (warp-collective).
 __device__ __forceinline__ void merge_lanes(float *kd, uint32_t *kc, const float *nd, const uint32_t *nc, int warp,
-                                           unsigned need, int &cnt, float &thr, float cap)
+                                     unsigned need, int &cnt, float &thr, float cap)
 {
 	const int lane = threadIdx.x & 31;
 	while (need) {
-		const int L = __ffs(need) - 1;
-		need &= need - 1u;
-		const int cl = __shfl_sync(0xffffffffu, cnt, L);
-		const float t = merge_row(kd, kc, nd, nc, warp * 32 + L, cl);
-		if (lane == L) {
-			thr = fminf(t, cap);
-			cnt = 0;
+		int row[kMerge], n[kMerge];
+		float last[kMerge];
+#pragma unroll
+		for (int q = 0; q < kMerge; q++) {
+			const int L = need ? __ffs(need) - 1 : row[0] - warp * 32;
+			need &= need - 1u;
+			row[q] = warp * 32 + L;
+			n[q] = __shfl_sync(0xffffffffu, cnt, L);
 		}
+		merge_rows(kd, kc, nd, nc, row, n, last);
+		__syncwarp();
+#pragma unroll
+		for (int q = 0; q < kMerge; q++)
+			if (lane == row[q] - warp * 32) {
+				thr = fminf(last[q], cap);
+				cnt = 0;
+			}
 	}
 }
 
@@ -271,8 +316,8 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 	if (tid == 0) {
 		umma::mbar_init(&mma_done[0], 1);
 		umma::mbar_init(&mma_done[1], 1);
-		umma::mbar_init(&qn_full[0], 128);
-		umma::mbar_init(&qn_full[1], 128);
+		umma::mbar_init(&qn_full[0], 256);
+		umma::mbar_init(&qn_full[1], 256);
 		umma::mbar_init(&epi_done[0], 4);
 		umma::mbar_init(&epi_done[1], 4);
 		umma::mbar_init_fence();
@@ -379,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 		} else {
 			// A operand: the 128 reference patches, centred FP16
 			const int pt = tid - 128;
-			for (int it = pt; it < kRefs * 4; it += 128) {
+			for (int it = pt; it < kRefs * 4; it += 256) {
 				const int r = it >> 2, part = it & 3;
 				float s = 0.f, er = 0.f;
 				if (s_g[r] >= 0) {
@@ -466,21 +511,22 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 						umma::fence_after_sync();
 						const float *qn = qnc + b * kN;
 						const int n0 = ch * kN;
+						int row0 = n0 / UW, col0 = n0 - row0 * UW - 32;
 						for (int grp = 0; grp < kN / 32; grp++) {
 							const int g0c = n0 + grp * 32;
 							if (g0c >= nu) break;
-							const int row0 = g0c / UW, col0 = g0c - row0 * UW;
+							// the run of 32 starts at column col0 of the union's row row0; the bits of
+							// a row's part of the reference's window, shifted in from either side
+							col0 += 32;
+							while (col0 >= UW) {
+								col0 -= UW;
+								row0++;
+							}
 							uint32_t wmask = 0;
-							if (valid && wnx > 0) {
-								for (int k = 0;; k++) {
-									const int cs = k * UW - col0;
-									if (cs >= 32) break;
-									if ((unsigned)(row0 + k - ly0) < (unsigned)wny) {
-										const int lo = max(0, cs + lx0), hi = min(32, cs + lx0 + wnx);
-										if (lo < hi)
-											wmask |= (hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u)) & ~((1u << lo) - 1u);
-									}
-								}
+							for (int cs = -col0, y = row0 - ly0; cs < 32; cs += UW, y++) {
+								const int lo = min(max(cs + lx0, 0), 32), hi = min(max(cs + lx0 + wnx, 0), 32);
+								const uint32_t m = (uint32_t)((1ull << hi) - 1ull) & ~(uint32_t)((1ull << lo) - 1ull);
+								wmask |= (unsigned)y < (unsigned)wny ? m : 0u;
 							}
 							if (!__any_sync(0xffffffffu, wmask)) continue;
 							uint32_t acc[32];
@@ -497,14 +543,18 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 								key[4 * c4 + 2] = fmaf(-2.f, __uint_as_float(acc[4 * c4 + 2]), q.z);
 								key[4 * c4 + 3] = fmaf(-2.f, __uint_as_float(acc[4 * c4 + 3]), q.w);
 							}
+							uint32_t h4[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-							for (int c = 0; c < 32; c++)
-								if (key[c] < thr) hits |= 1u << c;
-							hits &= wmask;
+							for (int c = 0; c < 8; c++)
+#pragma unroll
+								for (int q = 0; q < 4; q++) h4[q] |= key[8 * q + c] < thr ? 1u << (8 * q + c) : 0u;
+							hits = ((h4[0] | h4[1]) | (h4[2] | h4[3])) & wmask;
 							if (!__any_sync(0xffffffffu, hits)) continue;
 							// the hits join the reference's newcomers (candidate = frame << 16 |
-							// position in the frame's union), one per lane and round; a full
-							// list is merged into the kept 32 by the whole warp
+							// position in the frame's union), every lane at its own pace; lists
+							// without room for them are merged into the kept 32 by the whole
+							// warp first.  (A hit that the merge's new threshold excludes drops
+							// out in the next merge.)
 							if (hits) {
 #pragma unroll
 								for (int c4 = 0; c4 < 8; c4++)
@@ -512,20 +562,16 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 										make_float4(key[4 * c4], key[4 * c4 + 1], key[4 * c4 + 2], key[4 * c4 + 3]);
 							}
 							const uint32_t cbase = ((uint32_t)ii << 16) | (uint32_t)g0c;
-							while (__any_sync(0xffffffffu, hits)) {
-								if (hits) {
-									const int c = __ffs(hits) - 1;
-									hits &= hits - 1u;
-									const float d = mydv[c];
-									if (d < thr) {
-										nd[r * kLs + cnt] = d;
-										nc[r * kLs + cnt] = cbase + (uint32_t)c;
-										cnt++;
-									}
-								}
-								const unsigned full = __ballot_sync(0xffffffffu, cnt == kTop);
-								if (full) merge_lanes(kd, kc, nd, nc, warp, full, cnt, thr, cap);
+							const unsigned full = __ballot_sync(0xffffffffu, cnt + __popc(hits) > kTop);
+							if (full) merge_lanes(kd, kc, nd, nc, warp, full | __ballot_sync(0xffffffffu, cnt >= kMergeFrom), cnt, thr, cap);
+							while (hits) {
+								const int c = __ffs(hits) - 1;
+								hits &= hits - 1u;
+								nd[r * kLs + cnt] = mydv[c];
+								nc[r * kLs + cnt] = cbase + (uint32_t)c;
+								cnt++;
 							}
+							__syncwarp();
 						}
 						umma::fence_before_sync();
 						__syncwarp();
@@ -544,18 +590,18 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 					const int pitch = ((UW + PX + 2) + 1) & ~1;
 					const int wh = UH + PX - 1, ww = UW + PX - 1;
 					// the previous frame's chunks are all built: the window can go
-					asm volatile("bar.sync 1, 128;" ::: "memory");
+					asm volatile("bar.sync 1, 256;" ::: "memory");
 					// sixteen rows per warp in flight: loads first, then conversions
 					{
 						float em = 0.f;
 						const int nrow = PT * wh;
 						for (int x2 = lane; 2 * x2 < ww; x2 += 32) {
 							const bool two = 2 * x2 + 1 < ww;
-							for (int r0 = pw; r0 < nrow; r0 += 64) {
+							for (int r0 = pw; r0 < nrow; r0 += 128) {
 								float v0[16], v1[16];
 #pragma unroll
 								for (int k = 0; k < 16; k++) {
-									const int row = r0 + 4 * k;
+									const int row = r0 + 8 * k;
 									v0[k] = v1[k] = 0.f;
 									if (row < nrow) {
 										const int ht = row / wh, y = row - ht * wh;
@@ -566,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 								}
 #pragma unroll
 								for (int k = 0; k < 16; k++) {
-									const int row = r0 + 4 * k;
+									const int row = r0 + 8 * k;
 									if (row < nrow) {
 										const float a0 = v0[k] - centre, a1 = two ? v1[k] - centre : 0.f;
 										if (!(fabsf(a0) < 60000.f && fabsf(a1) < 60000.f)) s_bad = 1;
@@ -582,7 +628,7 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 						for (int o = 16; o > 0; o >>= 1) em = fmaxf(em, __shfl_xor_sync(0xffffffffu, em, o));
 						if (lane == 0) atomicMax(&s_emax, __float_as_int(em));
 					}
-					asm volatile("bar.sync 1, 128;" ::: "memory");
+					asm volatile("bar.sync 1, 256;" ::: "memory");
 					const int nu = UW * UH;
 					for (int ch = 0; ch < s_nch[ii]; ch++, jchunk++) {
 						const int b = jchunk & 1;
@@ -593,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 						const int n0 = ch * kN;
 						// lanes: candidate (lane & 7) of an 8-candidate run, part (lane >> 3)
 						const int part = lane >> 3;
-						for (int run = pw; run < kN / 8; run += 4) {
+						for (int run = pw; run < kN / 8; run += 8) {
 							const int n = run * 8 + (lane & 7);
 							const int nn = n0 + n;
 							float s = 0.f;
@@ -614,7 +660,7 @@ __global__ void __launch_bounds__(kThreads, 1) search_tc_kernel(Image src, StepP
 						}
 						umma::fence_proxy_async();
 						umma::mbar_arrive(&qn_full[b]);
-						asm volatile("bar.sync 1, 128;" ::: "memory");
+						asm volatile("bar.sync 1, 256;" ::: "memory");
 						if (pt == 0) {
 							umma::fence_after_sync();
 							const uint32_t a0 = umma::smem_u32(sA), b0 = umma::smem_u32(dst);
