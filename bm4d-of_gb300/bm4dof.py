@@ -580,8 +580,8 @@ class Context:
         if v.ndim == 4:
             v = np.ascontiguousarray(v[:, 0])
         F, H, W = v.shape
-        ff = np.zeros((F, 2, H, W), np.float32)
-        bf = np.zeros((F, 2, H, W), np.float32)
+        ff = np.empty((F, 2, H, W), np.float32)   # (written whole; the library maps its pages)
+        bf = np.empty((F, 2, H, W), np.float32)
         p = params or self.tvl1_params()
         _check(load().bm4dof_tvl1_video(self._h, C.c_void_p(v.ctypes.data), W, H, F, C.byref(p),
                                         C.c_void_p(ff.ctypes.data), C.c_void_p(bf.ctypes.data), 0))
