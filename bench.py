@@ -48,9 +48,9 @@ WORKLOADS = {
 CLI = dict(px1=4, px2=4, pt1=4, pt2=4, wx1=21, wx2=21, np1=16, np2=16, b1=3.0)
 METRIC = "megapixel-frames/s at 1 GPU, plain vs learned/mixed at ≤0.05 dB PSNR loss"
 UNIT = "MPF/s"
-# ncu dram__bytes_read + dram__bytes_write of one step-1 search_kernel launch on
-# 480x272x12 (one --set full capture of the small workload)
-SEARCH_TRAFFIC_SMALL = 12.04e6 + 7.60e6
+# ncu dram__bytes_read + dram__bytes_write of one step-1 search_block_kernel
+# launch on 480x272x12 (one --set full capture of the small workload)
+SEARCH_TRAFFIC_SMALL = 12.15e6 + 0.18e6
 # CPU sample (crop of the same workload) for the host-core baseline: 12
 # frames, so that every reference patch has the full 9-frame search range it
 # has in the long video
@@ -439,13 +439,14 @@ def main():
 
     if rank != 0:
         return 0
-    # roofline of the dominant kernel (patch search): algorithmic FP32
-    # operations (one subtract, one multiply, one add per patch element per
-    # candidate) over the measured launch duration
+    # roofline of the dominant kernel (patch search by 2x2 blocks of groups): FP32
+    # lane operations -- 36 squared differences (a subtraction and a multiply-add)
+    # per patch frame and candidate serve four groups -- over the measured launch
+    # duration
     whf = W * H * F
     groups = [round(r * whf / 100.0) for r in ratios]
     ncand = 21 * 21 * 9
-    flops_per_launch = statistics.mean(g * 3 * 64 * ncand for g in groups)
+    flops_per_launch = statistics.mean(g * 2 * 36 * 4 / 4 * ncand for g in groups)
     launch_ms = statistics.mean(searches) / 2.0
     achieved = flops_per_launch / (launch_ms / 1e3) / 1e12
     # the search's instruction mix timed alone on this GPU (registers only,
@@ -463,12 +464,12 @@ def main():
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
                      # DRAM bytes per launch: ncu capture of the 480x272x12 step-1 launch
-                     # (12.04 MB read + 7.60 MB written), scaled by the pixel count
+                     # (12.15 MB read + 0.18 MB written), scaled by the pixel count
                      "traffic": SEARCH_TRAFFIC_SMALL * (W * H * F) / (480 * 272 * 12),
-                     "traffic_source": "ncu dram__bytes_read+write of search_kernel on 480x272x12, "
+                     "traffic_source": "ncu dram__bytes_read+write of search_block_kernel on 480x272x12, "
                                        "scaled by pixels (the frames and flows, read about once)",
-                     "kernel": "search_kernel",
-                     "peak_source": "measured on this GPU by bm4dof_fp32_mix_rate: the exact search's FP32 "
+                     "kernel": "search_block_kernel",
+                     "peak_source": "measured on this GPU by bm4dof_fp32_mix_rate: the per-group search's FP32 "
                                     "instruction mix (packed sub/mul.rn.f32x2 + scalar adds) from registers, "
                                     "3 ops per element (MEASURED_PEAKS.json has HBM and bf16 tensor peaks only)",
                      "nominal_fp32_tops": nominal, "frac_of_nominal": achieved / nominal},
