@@ -927,6 +927,7 @@ cudaError_t tvl1_flow(const float *I0, const float *I1, int nx, int ny, int npai
 	const int nscales = pr.nscales;
 	const int fscale = std::min(pr.fscale, nscales);
 	const int m = mirrored ? npairs / 2 : npairs;   // images on each side
+	if (2 * (long long)m > 65535) { why = "too many frame pairs for one cooperative launch"; return cudaErrorInvalidValue; }
 	std::vector<int> NX(nscales), NY(nscales);
 	std::vector<float *> img(nscales), lu(nscales), lv(nscales);   // img: the m first images, the m second ones
 	NX[0] = nx;
