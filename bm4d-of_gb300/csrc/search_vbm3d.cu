@@ -256,10 +256,13 @@ __device__ bool half_select(const float *d, int n, int K, bool nan, float *od, i
 // Squared distances of the reference patch (ref, `reps` copies of channel 0
 // at stride spc) to the patches at p0 and p1 (channel 0 of each candidate's
 // first row and frame), terms in the reference's order; the two sums run
-// interleaved so that each hides the other's add latency.
+// interleaved so that each hides the other's add latency.  A lane without a
+// second candidate (two is false) leaves its loads out, which the L1 data path
+// feels (8x8, 720x576x3x14: 14.8 -> 13.9 ms); not with 4x4x4 patches, whose 64
+// registers have no room for the predicate's cost (25.3 -> 26.6).
 template <int PX, int PT>
 __device__ __forceinline__ void patch_distance2(const float *p0, const float *p1, size_t rpitch, size_t tpitch,
-                                                const float *ref, int reps, int px_rt, int pt_rt, float &a0,
+                                                const float *ref, int reps, int px_rt, int pt_rt, bool two, float &a0,
                                                 float &a1)
 {
 	// compile-time extents when the shape is a template argument (full
@@ -293,7 +296,7 @@ __device__ __forceinline__ void patch_distance2(const float *p0, const float *p1
 				for (int xx = 0; xx < (PX > 0 ? PX : px); xx++) {
 					const float rv = VEC ? rrow[xx % QV] : rf[xx];
 					float m0, m1;
-					sqdiff2(rv, rv, __ldg(p0 + off + xx), __ldg(p1 + off + xx), m0, m1);
+					sqdiff2(rv, rv, __ldg(p0 + off + xx), PX == 4 || two ? __ldg(p1 + off + xx) : 0.f, m0, m1);
 					a0 = __fadd_rn(a0, m0);
 					a1 = __fadd_rn(a1, m1);
 				}
@@ -304,10 +307,11 @@ __device__ __forceinline__ void patch_distance2(const float *p0, const float *p1
 
 // The same for reps > 1: the terms of the later passes are those of the first,
 // kept in registers, so a later pass is the additions alone.  (A call: one copy
-// of its 700 instructions for the places that need it.)
+// of its 700 instructions for the places that need it.  Second loads left out:
+// 7x7 2.84 -> 2.67 ms on 480x320x3x8, 8x8 13.9 -> 14.3 on 720x576x3x14.)
 template <int PX, int PT>
 __device__ __noinline__ float2 patch_distance2_reps(const float *p0, const float *p1, size_t rpitch, size_t tpitch,
-                                                    const float *ref, int reps)
+                                                    const float *ref, int reps, bool two)
 {
 	constexpr int N = PX * PX * PT;
 	float m0[N], m1[N], a0 = 0.f, a1 = 0.f;
@@ -320,7 +324,7 @@ __device__ __noinline__ float2 patch_distance2_reps(const float *p0, const float
 			for (int xx = 0; xx < PX; xx++) {
 				const int k = (tt * PX + yy) * PX + xx;
 				const float rv = ref[k];
-				sqdiff2(rv, rv, __ldg(p0 + off + xx), __ldg(p1 + off + xx), m0[k], m1[k]);
+				sqdiff2(rv, rv, __ldg(p0 + off + xx), PX == 8 || two ? __ldg(p1 + off + xx) : 0.f, m0[k], m1[k]);
 				a0 = __fadd_rn(a0, m0[k]);
 				a1 = __fadd_rn(a1, m1[k]);
 			}
@@ -337,13 +341,13 @@ __device__ __noinline__ float2 patch_distance2_reps(const float *p0, const float
 
 template <int PX, int PT, bool REPS>
 __device__ __forceinline__ float2 pair_distance(const float *p0, const float *p1, size_t rpitch, size_t tpitch,
-                                                const float *ref, int reps, int px, int pt)
+                                                const float *ref, int reps, int px, int pt, bool two)
 {
 	if constexpr (REPS) {
-		return patch_distance2_reps<PX, PT>(p0, p1, rpitch, tpitch, ref, reps);
+		return patch_distance2_reps<PX, PT>(p0, p1, rpitch, tpitch, ref, reps, two);
 	} else {
 		float a0, a1;
-		patch_distance2<PX, PT>(p0, p1, rpitch, tpitch, ref, reps, px, pt, a0, a1);
+		patch_distance2<PX, PT>(p0, p1, rpitch, tpitch, ref, reps, px, pt, two, a0, a1);
 		return make_float2(a0, a1);
 	}
 }
@@ -438,7 +442,7 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 					const int qx = lane < npf ? (int)(q % (uint32_t)T.w) : x,
 					          qy = lane < npf ? (int)(q / (uint32_t)T.w % (uint32_t)T.h) : y;
 					const float *qp = src.p + src.at(T.ox + qx, T.oy + qy, qt, 0);
-					float2 d = pair_distance<PX, PT, REPS>(qp, qp, rpitch, tpitch, ref, a.reps, px, sp.pt);
+					float2 d = pair_distance<PX, PT, REPS>(qp, qp, rpitch, tpitch, ref, a.reps, px, sp.pt, false);
 					if (qx == x && qy == y) d.x = __fsub_rn(d.x, sp.dsub_bias);
 					if (lane < npf) {
 						pool_d[lane] = d.x;
@@ -456,7 +460,7 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 						          qy0 = fy0 + y0, qy1 = fy0 + y1;
 						float2 d = pair_distance<PX, PT, REPS>(src.p + src.at(T.ox + qx0, T.oy + qy0, qt, 0),
 						                                       src.p + src.at(T.ox + qx1, T.oy + qy1, qt, 0), rpitch, tpitch,
-						                                       ref, a.reps, px, sp.pt);
+						                                       ref, a.reps, px, sp.pt, c1 != c);
 						if (qx0 == x && qy0 == y) d.x = __fsub_rn(d.x, sp.dsub_bias);
 						if (qx1 == x && qy1 == y) d.y = __fsub_rn(d.y, sp.dsub_bias);
 						nan |= d.x != d.x || d.y != d.y;
@@ -516,7 +520,7 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 					const int qx1 = (int)(q1 & 0xffffu), qy1 = (int)(q1 >> 16);
 					const float2 d = pair_distance<PX, PT, REPS>(src.p + src.at(T.ox + qx0, T.oy + qy0, qt, 0),
 					                                             src.p + src.at(T.ox + qx1, T.oy + qy1, qt, 0), rpitch,
-					                                             tpitch, ref, a.reps, px, sp.pt);
+					                                             tpitch, ref, a.reps, px, sp.pt, two);
 					float d0 = d.x, d1 = d.y;
 					if (qx0 == x && qy0 == y) d0 = __fsub_rn(d0, sp.dsub_bias);
 					if (qx1 == x && qy1 == y) d1 = __fsub_rn(d1, sp.dsub_bias);
@@ -605,7 +609,7 @@ search_vbm3d_kernel(Image src, Image ffl, Image bfl, StepParams sp, VArgs a)
 					const int qx1 = (int)(q1 & 0xffffu), qy1 = (int)(q1 >> 16);
 					const float2 d = pair_distance<PX, PT, REPS>(
 					    src.p + src.at(T.ox + qx0, T.oy + qy0, s0 ? t - k : t + k, 0),
-					    src.p + src.at(T.ox + qx1, T.oy + qy1, s1 ? t - k : t + k, 0), rpitch, tpitch, ref, a.reps, px, sp.pt);
+					    src.p + src.at(T.ox + qx1, T.oy + qy1, s1 ? t - k : t + k, 0), rpitch, tpitch, ref, a.reps, px, sp.pt, two);
 					float d0 = d.x, d1 = d.y;
 					if (qx0 == x && qy0 == y) d0 = __fsub_rn(d0, sp.dsub_bias);
 					if (qx1 == x && qy1 == y) d1 = __fsub_rn(d1, sp.dsub_bias);
@@ -754,8 +758,8 @@ cudaError_t launch_search_vbm3d(const Image &src, const Image &ffl, const Image 
 	}();
 	// (repeated distances: 168 registers for the 128 terms of two candidates).
 	// 720x576x3x14 with the default parameters (8x8, 7x7 windows; reps 1, then 3):
-	// 21.3 ms with strips and every pass computed again, 14.6 now; 480x320x3x8 at
-	// sigma 20 (7x7 in step 2, without a template of its own before) 6.5 -> 3.0.
+	// 21.3 ms with strips and every pass computed again, 13.9 now; 480x320x3x8 at
+	// sigma 20 (7x7 in step 2, without a template of its own before) 6.5 -> 2.7.
 	if (sp.px == 4 && sp.pt == 4) {
 		if (reps > 1) return launch_t<4, 4, 3, true>(src, ffl, bfl, sp, a, nsm, st);
 		if (minb == 4) return launch_t<4, 4, 4>(src, ffl, bfl, sp, a, nsm, st);
