@@ -25,6 +25,10 @@
 //     reference's order; what is still equal then (std::partial_sort's heap
 //     decides) is left to search.cu's kernel, as are groups whose list
 //     overflows and sources with values that are not finite.
+//   * Blocks that do not pay.  The four windows of a block follow their own
+//     flows; where those differ the block covers the windows' union, which may
+//     cost more than the four windows one by one.  Such a block is left to
+//     search.cu's kernel before it is computed (pays_off).
 //
 // What bounds it: issue slots and L1.  Per displacement of a block (four
 // distances) of 4x4x4 patches with S = 2 a warp issues 168 packed or scalar FP32
@@ -221,6 +225,22 @@ struct BlockArgs {
 
 __device__ __forceinline__ unsigned redux_min(unsigned v) { return __reduce_min_sync(0xffffffffu, v); }
 
+// Whether a block of `rounds` rounds of 32 columns is cheaper here than four
+// groups with `cand` candidates in all in search.cu's kernel.  Nanoseconds of the
+// whole GPU, fitted to both kernels' times (854x480x8, windows of 9, 21 and 39; 8x8
+// and 7x7 also 7x7 windows): a block takes 13 and 0.025 (4x4x4) or 0.036 a round
+// and pixel of the block, a group 10 (4x4x4) or 50 and 0.011 a candidate and
+// channel.  4x4x4, step 2, 21x21 windows over 5 frames: 49 against 137, so the
+// rounds may rise from 10 to 34.  Without the rule flows with a noise of 8 / 20
+// pixels took 21.9 / 52.2 ms (480x272x10, both steps) where the per-group kernel
+// takes 15.0 / 16.0.
+template <int P, int S, int PT>
+__device__ __forceinline__ bool pays_off(int rounds, int cand, int chn)
+{
+	constexpr float kRound = (P == 4 ? 0.025f : 0.036f) * PT * (P + S) * (P + S), kGroup = P == 4 ? 10.f : 50.f;
+	return 13.f + kRound * (float)(rounds * chn) <= 4.f * kGroup + 0.011f * (float)(cand * chn);
+}
+
 constexpr float kTiny = 1e-35f;        // below this the products may underflow
 constexpr float kMaxFinite = 3.0e38f;
 
@@ -357,8 +377,11 @@ search_block_kernel(Image src, StepParams sp, BlockArgs a)
 		int K[4];
 #pragma unroll
 		for (int k = 0; k < 4; k++) K[k] = min(sp.np, __reduce_add_sync(0xffffffffu, cand[k]));
+		// (in one condition with the next: another exit here costs the main loop registers)
+		wide |= !pays_off<P, S, PT>((nitems + 31) / 32, __reduce_add_sync(0xffffffffu, cand[0] + cand[1] + cand[2] + cand[3]) *
+		                                                (4 / (__popc(have) * __popc(havey))), chn);
 		if (__any_sync(0xffffffffu, wide) || nitems > 32 * kMaxRounds) {
-			// windows far apart (a motion boundary with a large jump)
+			// windows far apart: a motion boundary, a rough flow
 			if (a.glist && lane < 4 && exists(lane)) a.glist[atomicAdd(a.gcount, 1u)] = (uint32_t)group(lane);
 			continue;
 		}
