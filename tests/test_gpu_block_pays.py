@@ -48,3 +48,20 @@ def test_gpu_blocks_under_rough_flows(gpulib, gpuctx, noise, cli):
     ff, bf = rng.normal(0, noise, (2, F, 2, H, W))
     blocks, groups = compare(gpulib, gpuctx, nz, ff, bf, cli, 20.0)
     assert blocks <= 1.2 * groups, (blocks, groups)
+
+
+# exact ties in every group: before the rule 1.4 times the per-group kernel's
+# time; with it the look at the block's pixels more
+def test_gpu_blocks_on_flat_frames(gpulib, gpuctx):
+    nz = np.full((12, 1, 360, 640), 100.0, np.float32)
+    blocks, groups = compare(gpulib, gpuctx, nz, None, None, P4, 20.0)
+    assert blocks <= 1.2 * groups, (blocks, groups)
+
+
+# half the frame flat: blocks are computed again where they pay
+def test_gpu_blocks_on_half_flat_frames(gpulib, gpuctx):
+    rng = np.random.default_rng(3)
+    nz = np.full((12, 1, 360, 640), 100.0, np.float32)
+    nz[..., 320:] += rng.normal(0, 20, (12, 1, 360, 320)).astype(np.float32)
+    blocks, groups = compare(gpulib, gpuctx, nz, None, None, P4, 20.0)
+    assert blocks <= 1.2 * groups, (blocks, groups)
