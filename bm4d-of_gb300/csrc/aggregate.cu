@@ -390,24 +390,37 @@ __global__ void bin_alloc_kernel(unsigned nbins, const unsigned *__restrict__ cn
 	}
 }
 
-// Adds a 4-row column of terms w * v to the rows R .. R + 3 of a lane's 8 sums.  The
+// Adds a column of PX terms w * v to the rows R .. R + PX - 1 of a lane's 8 sums.  The
 // markers keep the compiler from merging the cases of R into one that indexes
 // the sums dynamically, which would put them in local memory.
-template <int R, int CC>
-__device__ __forceinline__ void add_rows(float (&a)[8][CC], float (&wa)[8], const float4 (&v)[CC], float w)
+template <int R, int PX, int CC>
+__device__ __forceinline__ void add_rows(float (&a)[8][CC], float (&wa)[8], const float (&v)[CC][PX], float w)
 {
 	asm volatile("" ::"n"(R));
 #pragma unroll
-	for (int h = 0; h < 4; h++)
+	for (int h = 0; h < PX; h++)
 		if (R + h >= 0 && R + h < 8) {
 #pragma unroll
-			for (int c = 0; c < CC; c++) {
-				const float t = h == 0 ? v[c].x : h == 1 ? v[c].y : h == 2 ? v[c].z : v[c].w;
-				a[(R + h) & 7][c] = __fadd_rn(a[(R + h) & 7][c], __fmul_rn(w, t));
-			}
+			for (int c = 0; c < CC; c++) a[(R + h) & 7][c] = __fadd_rn(a[(R + h) & 7][c], __fmul_rn(w, v[c][h]));
 			wa[(R + h) & 7] = __fadd_rn(wa[(R + h) & 7], w);
 		}
 	asm volatile("" ::"n"(R + 16));
+}
+
+__device__ __forceinline__ void load_column(const float *p, float (&v)[4])
+{
+	const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+	v[0] = q.x;
+	v[1] = q.y;
+	v[2] = q.z;
+	v[3] = q.w;
+}
+
+__device__ __forceinline__ void load_column(const float *p, float (&v)[2])
+{
+	const float2 q = __ldg(reinterpret_cast<const float2 *>(p));
+	v[0] = q.x;
+	v[1] = q.y;
 }
 
 // Ordered gather of one bin per CTA at a time.
@@ -424,10 +437,11 @@ __device__ __forceinline__ void add_rows(float (&a)[8][CC], float (&wa)[8], cons
 // in registers, and adds a slot's terms to the pixels the slot covers, slots in
 // order: the order of the reference's scatter loop for every pixel.  Only the
 // terms a lane needs are loaded, each once; U slots' loads are in flight before
-// the first is added.  4x4 patches: a lane owns one column of 8 pixels of one
-// of four frames; the patch's four terms of that column and frame are one
-// 16-byte load (term_of orders them so), and the rows they fall on are the same
-// for the whole warp.  Other patches: a lane owns pixels (x, y) and (x, y + 4).
+// the first is added.  4x4 patches and 2x2 ones of several frames: a lane owns one column of 8
+// pixels of one of four frames; the patch's terms of that column and frame are one 16- or
+// 8-byte load (term_of orders them so), and the rows they fall on are the same
+// for the whole warp.  Other patches: a lane owns pixels (x, y) and (x, y + 4); by
+// that mapping 2x2x4 patches took 11.3 ms (240x180x8), by columns 6.3.
 template <int PX, int BT, int CC, int U>
 __global__ void __launch_bounds__(kGatherThreads)
 bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, long long ga,
@@ -437,7 +451,7 @@ bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, lon
                   const unsigned *__restrict__ list, float *__restrict__ acc, float *__restrict__ wacc)
 {
 	constexpr int kBitWords = BT == 1 ? 512 : 2048;
-	constexpr bool kColumn = PX == 4;
+	constexpr bool kColumn = PX == 4 || PX == 2;
 	static_assert(!kColumn || BT == 4, "a lane's frame is one of four");
 	__shared__ unsigned s_bits[kBitWords];
 	__shared__ uint4 s_ent[kEntCap];         // slot, place relative to the bin, weight
@@ -587,13 +601,13 @@ bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, lon
 						unsigned m = __ballot_sync(0xffffffffu, hit);
 						if constexpr (kColumn) {
 							while (m) {
-								float4 v[U][CC];
+								float v[U][CC][PX ? PX : 1];
 								float wt[U];
 								int row[U];
 								bool ok[U];
 #pragma unroll
 								for (int u = 0; u < U; u++) {
-									row[u] = -4;
+									row[u] = -PX;
 									ok[u] = false;
 									if (!m) continue;
 									const uint4 q = s_ent[e + __ffs(m) - 1];
@@ -601,28 +615,28 @@ bin_gather_kernel(const Tile *__restrict__ tiles, int ntiles, StepParams sp, lon
 									const unsigned dx = (unsigned)(x - X0 + 8) - (q.y & 255u);
 									const unsigned dt = (unsigned)((lane >> 3) + 16) - (q.y >> 16);
 									row[u] = (int)(q.y >> 8 & 255u) - 8 + Y0 - qy;
-									ok[u] = dx < 4u && dt < (unsigned)pt;
+									ok[u] = dx < (unsigned)PX && dt < (unsigned)pt;
 									wt[u] = __uint_as_float(q.z);   // no window for these patches
-									const float *col = vals + (size_t)q.x * (spc * CC) + (dt * 4u + dx) * 4u;
+									const float *col = vals + (size_t)q.x * (spc * CC) + (dt * PX + dx) * PX;
 #pragma unroll
 									for (int c = 0; c < CC; c++)
-										if (ok[u]) v[u][c] = __ldg(reinterpret_cast<const float4 *>(col + c * spc));
+										if (ok[u]) load_column(col + c * spc, v[u][c]);
 								}
 #pragma unroll
 								for (int u = 0; u < U; u++)
 									if (ok[u]) {
 										switch (row[u]) {   // the same for the whole warp
-										case -3: add_rows<-3>(a, wa, v[u], wt[u]); break;
-										case -2: add_rows<-2>(a, wa, v[u], wt[u]); break;
-										case -1: add_rows<-1>(a, wa, v[u], wt[u]); break;
-										case 0: add_rows<0>(a, wa, v[u], wt[u]); break;
-										case 1: add_rows<1>(a, wa, v[u], wt[u]); break;
-										case 2: add_rows<2>(a, wa, v[u], wt[u]); break;
-										case 3: add_rows<3>(a, wa, v[u], wt[u]); break;
-										case 4: add_rows<4>(a, wa, v[u], wt[u]); break;
-										case 5: add_rows<5>(a, wa, v[u], wt[u]); break;
-										case 6: add_rows<6>(a, wa, v[u], wt[u]); break;
-										case 7: add_rows<7>(a, wa, v[u], wt[u]); break;
+										case -3: add_rows<-3, PX>(a, wa, v[u], wt[u]); break;
+										case -2: add_rows<-2, PX>(a, wa, v[u], wt[u]); break;
+										case -1: add_rows<-1, PX>(a, wa, v[u], wt[u]); break;
+										case 0: add_rows<0, PX>(a, wa, v[u], wt[u]); break;
+										case 1: add_rows<1, PX>(a, wa, v[u], wt[u]); break;
+										case 2: add_rows<2, PX>(a, wa, v[u], wt[u]); break;
+										case 3: add_rows<3, PX>(a, wa, v[u], wt[u]); break;
+										case 4: add_rows<4, PX>(a, wa, v[u], wt[u]); break;
+										case 5: add_rows<5, PX>(a, wa, v[u], wt[u]); break;
+										case 6: add_rows<6, PX>(a, wa, v[u], wt[u]); break;
+										case 7: add_rows<7, PX>(a, wa, v[u], wt[u]); break;
 										}
 									}
 							}
@@ -714,6 +728,7 @@ template <int CC, class... Args>
 cudaError_t gather_c(const StepParams &sp, Args... args)
 {
 	if (sp.px == 4) return sp.gather_depth == 2 && CC == 1 ? gather_t<4, 4, CC, CC == 1 ? 8 : 4>(args...) : gather_t<4, 4, CC, 4>(args...);
+	if (sp.px == 2 && sp.pt != 1) return gather_t<2, 4, CC, 4>(args...);
 	if (sp.pt != 1) return gather_t<0, 4, CC, 1>(args...);
 	if (sp.px == 7) return gather_t<7, 1, CC, CC == 1 ? 4 : 2>(args...);
 	if (sp.px == 8) return gather_t<8, 1, CC, CC == 1 ? 4 : 2>(args...);

@@ -67,13 +67,14 @@ struct StepParams {               // resolved parameters of one step
 
 // Aggregation terms of a chunk of groups: for slot s (one member of one
 // group), channel c and patch element p, the estimate ghat at
-// vals[(s * C + c) * spc + term_of(px, p)], and the member's weight w at
+// vals[(s * C + c) * spc + term_of(px, pt, p)], and the member's weight w at
 // wslot[s] (the gather forms (w * window[p]) * ghat itself).  4x4
-// patches hold each frame's elements column by column, so that the gather's
-// lanes read the four rows of a column with one load.
-__host__ __device__ __forceinline__ int term_of(int px, int p)
+// patches, and 2x2 ones of several frames, hold each frame's elements column by
+// column, so that the gather's lanes read the rows of a column with one load.
+__host__ __device__ __forceinline__ int term_of(int px, int pt, int p)
 {
-	return px == 4 ? (p & ~15) | (p & 3) << 2 | (p >> 2 & 3) : p;
+	return px == 4 ? (p & ~15) | (p & 3) << 2 | (p >> 2 & 3)
+	               : px == 2 && pt > 1 ? (p & ~3) | (p & 1) << 1 | (p >> 1 & 1) : p;
 }
 
 // Aggregation bins: pixels x frames of one tile.

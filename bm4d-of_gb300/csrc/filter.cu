@@ -257,7 +257,7 @@ filter_exact_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, in
 			for (int it = tid; it < ns * per; it += blockDim.x) {
 				const int n = it / per, r = it % per;
 				const int c = r / spc, p = r % spc;
-				vals[((slot0 + n) * C + c) * spc + term_of(px, p)] = Gn[r * nsp + n];
+				vals[((slot0 + n) * C + c) * spc + term_of(px, pt, p)] = Gn[r * nsp + n];
 			}
 			if (tid == 0) eq[g] = 1;
 			continue;
@@ -321,7 +321,7 @@ filter_exact_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, in
 		for (int it = tid; it < ns * per; it += blockDim.x) {
 			const int n = it / per, r = it % per;
 			const int c = r / spc, p = r % spc;
-			vals[((slot0 + n) * C + c) * spc + term_of(px, p)] = Gn[r * nsp + n];
+			vals[((slot0 + n) * C + c) * spc + term_of(px, pt, p)] = Gn[r * nsp + n];
 		}
 		if (tid < ns) wslot[slot0 + tid] = w;
 		if (tid == 0) { wgroup[g] = w; eq[g] = 0; }
@@ -690,7 +690,7 @@ filter_warp_kernel(Image noisy, Image basic, const Tile *__restrict__ tiles, int
 						// left as it is; its weights are set later (fixup_equal_kernel)
 						for (int i = 0; i < C * SPC && n < ns; i++) {
 							const int c = i / SPC, p = i % SPC;
-							vals[((slot0 + n) * C + c) * SPC + term_of(PX, p)] =
+							vals[((slot0 + n) * C + c) * SPC + term_of(PX, PT, p)] =
 							    __ldg(noisy.p + base + noisy.at(p % PX, p / PX % PX, p / (PX * PX), c));
 						}
 						if (n == 0) eq[g] = 1;

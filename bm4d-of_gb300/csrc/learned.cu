@@ -235,7 +235,7 @@ __device__ void group_body(const LearnedArgs &a, const StepParams &sp, long long
 	const long long slot0 = r * sp.np;
 #pragma unroll
 	for (int m = 0; m < NS; m++)
-		a.vals[(slot0 + m) * kSpc + term_of(sp.px, k)] = est[m];
+		a.vals[(slot0 + m) * kSpc + term_of(sp.px, sp.pt, k)] = est[m];
 	if (k < NS) a.wslot[slot0 + k] = wgt;
 }
 
@@ -539,7 +539,7 @@ learned_tc_kernel(LearnedArgs a, StepParams sp)
 		const int p = lane + 32 * h, ht = p / (px * px), hy = (p / px) % px, hx = p % px;
 		off[h] = (long long)a.noisy.at(hx, hy, ht, 0) - (long long)a.noisy.at(0, 0, 0, 0);
 	}
-	const int term[2] = {term_of(px, lane), term_of(px, lane + 32)};
+	const int term[2] = {term_of(px, sp.pt, lane), term_of(px, sp.pt, lane + 32)};
 	const long long first = a.ga + (long long)blockIdx.x * kTcWarps + warp, step = (long long)gridDim.x * kTcWarps;
 	int alive = 0, ns = 0;
 	uint32_t lin = 0;
