@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/bm4dof.h"
+#include "chunk.hpp"
 #include "internal.hpp"
 
 using namespace bm4dof;
@@ -61,8 +62,9 @@ struct bm4dof_ctx {
 	// mixed form: groups searched through the tensor-core pre-screen, and the
 	// ones it left to the exact search, over both steps of the last run
 	unsigned long long m_groups = 0, m_exact = 0, m_uncertified = 0;
-	size_t slot_budget = 0;   // bytes of per-chunk aggregation terms
-	bool fixed_budget = false;   // batched children: slot_budget set by the tuning
+	size_t chunk_bytes = 0;   // bytes of a chunk's terms, weights and bin lists
+	bool fixed_chunk = false;    // batched children: chunk_bytes set by the tuning
+	bool tight = false;          // a run has not fitted the memory limit with chunks of a quarter of it
 	bool no_marks = false;       // inside a graph capture: no timing events
 	int search_ctas = 0;         // per-group search: CTAs per SM (0: default)
 	int search_strip = 0;        // 7: per-group search (0, 21: default)
@@ -444,22 +446,15 @@ bm4dof_status hbuf(bm4dof_ctx *ctx, const std::string &name, size_t bytes, unsig
 	return BM4DOF_OK;
 }
 
-// Bytes of aggregation terms per chunk: 16 GB, BM4DOF_SLOT_MB when set (a
-// decimal number of MiB, fractions allowed), at most half of the device
-// memory this context could use.
-void set_budget(bm4dof_ctx *ctx)
+// The size of a single run's chunks (chunk.hpp); BM4DOF_SLOT_MB is a decimal
+// number of MiB, fractions allowed.
+void set_chunk(bm4dof_ctx *ctx)
 {
-	if (ctx->fixed_budget) return;
-	size_t budget = (size_t)16384 << 20;
-	if (const char *env = std::getenv("BM4DOF_SLOT_MB")) {
-		const double mb = std::atof(env);
-		if (mb > 0.0) budget = (size_t)(mb * 1048576.0);
-	}
+	if (ctx->fixed_chunk) return;
+	const char *env = std::getenv("BM4DOF_SLOT_MB");
 	size_t freeb = 0, totalb = 0;
-	if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && budget > (freeb + ctx->held) / 2)
-		budget = (freeb + ctx->held) / 2;
-	if (ctx->mem_limit && budget > ctx->mem_limit / 4) budget = ctx->mem_limit / 4;
-	ctx->slot_budget = budget;
+	if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = 0;
+	ctx->chunk_bytes = chunk_bytes(env ? std::atof(env) : 0.0, freeb ? freeb + ctx->held : 0, ctx->mem_limit, ctx->tight);
 }
 
 std::string nm(int slot, const char *base) { return std::string(slot ? "s2_" : "s1_") + base; }
@@ -594,11 +589,7 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 		SBUF("paste_counts", kPasteRounds + 3, S.paste.counts);
 	}
 
-	// shared aggregation buffers; chunks of groups whose terms, weights and
-	// bin lists take at most an eighth of the slot budget (half of a batched
-	// sequence's, which is the smaller): with 2 GiB chunks a new context
-	// allocates 14 GiB less than with whole-budget ones, and the gather still
-	// sees thousands of bins per chunk
+	// shared aggregation buffers
 	if (pl.nbins > 0x7fffffffll) {
 		set_error("bm4dof: unsupported parameters: video too large");
 		return BM4DOF_ERR_UNSUPPORTED;
@@ -613,10 +604,7 @@ bm4dof_status prepare_step(bm4dof_ctx *ctx, int slot, int step, const bm4dof_par
 	const size_t per_group = (size_t)sp.np * ((size_t)C * sp.spc + 1 + (size_t)bin_entries_per_member(sp)) *
 	                             sizeof(float) +
 	                         (mode.learned ? (size_t)kMlpInPad * 2 + (size_t)kMlpOutN * 4 : 0);
-	const size_t budget = ctx->slot_budget / (ctx->fixed_budget ? 2 : 8);
-	long long chunk = std::max<long long>(1, (long long)(budget / per_group));
-	chunk = std::min<long long>(chunk, (1ll << 28) / sp.np);   // list positions fit 32 bits
-	chunk = std::min<long long>(chunk, std::max<long long>(1, G));
+	const long long chunk = chunk_groups(ctx->chunk_bytes, per_group, sp.np, bin_entries_per_member(sp), G);
 	S.chunk = chunk;
 	if (!mode.samples) {
 		DBUF("vals", (size_t)chunk * sp.np * C * sp.spc, S.d_vals);
@@ -877,7 +865,7 @@ bm4dof_ctx *make_child(bm4dof_ctx *parent)
 	c->nsm = parent->nsm;
 	c->st = nullptr;        // a branch stream of the parent
 	c->no_marks = true;
-	c->fixed_budget = true;
+	c->fixed_chunk = true;
 	return c;
 }
 
@@ -1054,8 +1042,7 @@ bm4dof_status validate_run(RunArgs &r, const char *who)
 	return BM4DOF_OK;
 }
 
-// Inputs, outputs and both steps allocated before any launch.
-bm4dof_status prepare_run(bm4dof_ctx *ctx, RunArgs &r)
+bm4dof_status allocate_run(bm4dof_ctx *ctx, RunArgs &r)
 {
 	const size_t P = (r.W + 7) / 8 * 8;
 	const size_t nv = P * r.H * r.C * r.F;
@@ -1079,6 +1066,29 @@ bm4dof_status prepare_run(bm4dof_ctx *ctx, RunArgs &r)
 			return e;
 	}
 	return BM4DOF_OK;
+}
+
+// Inputs, outputs and both steps allocated before any launch; with smaller chunks
+// where the memory limit leaves no room for the first size.
+bm4dof_status prepare_run(bm4dof_ctx *ctx, RunArgs &r)
+{
+	bm4dof_status e = allocate_run(ctx, r);
+	if (e != BM4DOF_ERR_NO_MEMORY || !ctx->mem_limit || ctx->tight || ctx->fixed_chunk) return e;
+	ctx->tight = true;
+	set_chunk(ctx);
+	clear_error();
+	e = allocate_run(ctx, r);
+	if (e != BM4DOF_ERR_NO_MEMORY) return e;
+	// the first attempt's chunk buffers may be what is in the way
+	for (const char *name : {"vals", "wslot", "bin_list", "lfeat", "lgain"}) {
+		DevBuf &b = ctx->bufs[name];
+		if (b.p) cudaFree(b.p);
+		ctx->held -= b.cap;
+		b.p = nullptr;
+		b.cap = 0;
+	}
+	clear_error();
+	return allocate_run(ctx, r);
 }
 
 // The whole run on the context's stream: uploads, both steps, downloads.
@@ -1217,7 +1227,7 @@ bm4dof_status bm4dof_run(bm4dof_ctx *ctx, const float *noisy, const float *fflow
 		CK(cudaEventCreate(&ctx->t_begin));
 		CK(cudaEventCreate(&ctx->t_end));
 	}
-	set_budget(ctx);
+	set_chunk(ctx);
 	ctx->whf = (float)(W * H * F);
 	if ((e = prepare_run(ctx, r)) != BM4DOF_OK) return e;
 	CK(cudaEventRecord(ctx->t_begin, ctx->st));
@@ -1268,6 +1278,7 @@ bm4dof_status bm4dof_set_memory_limit(bm4dof_ctx *ctx, size_t bytes)
 		return BM4DOF_ERR_ARGUMENT;
 	}
 	ctx->mem_limit = bytes;
+	ctx->tight = false;
 	return BM4DOF_OK;
 }
 
@@ -1315,7 +1326,7 @@ bm4dof_status bm4dof_process(bm4dof_ctx *ctx, const float *noisy, const float *f
 		CK(cudaEventCreate(&ctx->t_begin));
 		CK(cudaEventCreate(&ctx->t_end));
 	}
-	set_budget(ctx);
+	set_chunk(ctx);
 	ctx->whf = (float)(W * H * F);
 	if ((e = prepare_run(ctx, r)) != BM4DOF_OK) return e;
 	CK(cudaEventRecord(ctx->t_begin, ctx->st));
@@ -1394,14 +1405,14 @@ bm4dof_status run_batched(bm4dof_ctx *ctx, bm4dof_sequence *seqs, unsigned n, un
 		}
 		if (!X.fork) CK(cudaEventCreateWithFlags(&X.fork, cudaEventDisableTiming));
 		while (X.children.size() < n) X.children.push_back(make_child(ctx));
-		// every sequence holds its buffers for the whole graph: the chunk
-		// budgets of all of them together stay within half the device memory
-		size_t per_child = (size_t)(tu.slot_mb ? tu.slot_mb : 1024) << 20;
+		// every sequence holds its buffers for the whole graph: the chunks of all
+		// of them together stay within a quarter of the device memory
+		size_t per_child = tu.slot_mb ? (size_t)tu.slot_mb << 20 : kBatchChunkBytes;
 		{
 			size_t freeb = 0, totalb = 0, held = 0;
 			for (bm4dof_ctx *c : X.children) held += c->held;
 			if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess) {
-				const size_t cap = std::max<size_t>((size_t)64 << 20, (freeb + held) / 2 / n);
+				const size_t cap = std::max<size_t>((size_t)32 << 20, (freeb + held) / 4 / n);
 				per_child = std::min(per_child, cap);
 			}
 		}
@@ -1409,7 +1420,7 @@ bm4dof_status run_batched(bm4dof_ctx *ctx, bm4dof_sequence *seqs, unsigned n, un
 		for (unsigned i = 0; i < n; i++) {
 			bm4dof_ctx *c = X.children[i];
 			c->st = X.branches[i % nb];
-			c->slot_budget = per_child;
+			c->chunk_bytes = per_child;
 			c->search_ctas = tu.search_ctas;
 			c->search_strip = tu.search_strip;
 			c->gather_depth = tu.gather_depth;
@@ -1744,7 +1755,7 @@ bm4dof_status bm4dof_gain_samples(bm4dof_ctx *ctx, const float *noisy, const flo
 	SampleOut so = {feat, target, valid, cap, count};
 	RunMode mode;
 	mode.samples = &so;
-	set_budget(ctx);
+	set_chunk(ctx);
 	ctx->whf = (float)(W * H * F);
 	for (int pass = 0; pass < 2; pass++)
 		if ((s = prepare_step(ctx, 1, 2, *p2, W, H, 1, F, fflow != nullptr, nparts, mode)) != BM4DOF_OK) return s;

@@ -129,8 +129,9 @@ bm4dof_status bm4dof_get_stream(bm4dof_ctx *ctx, void **stream);
 
 /* Caps the device memory the context's buffers may hold (0: no cap, the
  * default).  A call that would need more fails with BM4DOF_ERR_NO_MEMORY and
- * a message naming the buffer; the context stays usable.  The chunk budget of
- * the aggregation terms shrinks with the cap.  Applies to the calls made on
+ * a message naming the buffer; the context stays usable.  The chunks of the
+ * aggregation shrink with the cap, to a quarter of it or, where the other buffers
+ * need the room, a 32nd.  Applies to the calls made on
  * this context (not to the private contexts of bm4dof_run_batched). */
 bm4dof_status bm4dof_set_memory_limit(bm4dof_ctx *ctx, size_t bytes);
 
@@ -286,8 +287,9 @@ typedef struct bm4dof_sequence {
 /* Launch shape of a batched run (bm4dof_autotune chooses one). */
 typedef struct bm4dof_tuning {
 	unsigned branches;     /* concurrent streams in the graph; 0: min(n, 16)     */
-	unsigned slot_mb;      /* per sequence: MB of aggregation terms per chunk
-	                          (the depth of group staging); 0: 1024              */
+	unsigned slot_mb;      /* per sequence: MB of aggregation terms, weights and
+	                          lists per chunk (the depth of group staging);
+	                          0: 512                                             */
 	unsigned search_ctas;  /* per-group exact search, CTAs per SM: 4 or 6; 0: 6  */
 	unsigned search_strip; /* 21 or 0: the exact search by blocks of 2 x 2
 	                          neighbouring patches where the patch shape and grid
@@ -302,8 +304,8 @@ typedef struct bm4dof_tuning {
 
 /* Denoises n sequences (flags: BM4DOF_MIXED_PRECISION, BM4DOF_LEARNED,
  * BM4DOF_VBM3D_SEARCH; the pointers are always device pointers).  tuning may
- * be NULL (defaults).  Each sequence's chunk budget is capped so that all the
- * sequences' buffers fit in half the device memory.  bm4dof_last_timings
+ * be NULL (defaults).  Each sequence's chunks are capped so that those of
+ * all sequences take at most a quarter of the device memory.  bm4dof_last_timings
  * reports the graph launch as ms[4]. */
 bm4dof_status bm4dof_run_batched(bm4dof_ctx *ctx, bm4dof_sequence *seqs, unsigned n, unsigned flags,
                                  const bm4dof_tuning *tuning);
