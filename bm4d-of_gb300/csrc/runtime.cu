@@ -22,6 +22,7 @@
 
 #include "../../include/bm4dof.h"
 #include "chunk.hpp"
+#include "host_pages.hpp"
 #include "internal.hpp"
 
 using namespace bm4dof;
@@ -1836,14 +1837,16 @@ void map_output(void *p, size_t bytes)
 		cudaGetLastError();
 		return;
 	}
-	if (at.type != cudaMemoryTypeUnregistered || bytes == 0) return;
-	volatile char *c = static_cast<volatile char *>(p);
-	for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
-	c[bytes - 1] = 0;
+	if (at.type == cudaMemoryTypeUnregistered) touch_pages(p, bytes);
 }
 
-bm4dof_status tvl1_timed_out()
+// Waits for the flow; an error leaves the caller's outputs as they were.
+bm4dof_status tvl1_wait(bm4dof_ctx *ctx, const int *d_timed_out)
 {
+	int timed_out = 0;
+	CK(cudaMemcpyAsync(&timed_out, d_timed_out, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+	CK(cudaStreamSynchronize(ctx->st));
+	if (!timed_out) return BM4DOF_OK;
 	set_error("bm4dof_tvl1: a barrier of the fixed-point iterations ran into its limit");
 	return BM4DOF_ERR_CUDA;
 }
@@ -1899,7 +1902,7 @@ bm4dof_status bm4dof_tvl1_pairs(bm4dof_ctx *ctx, const float *I0, const float *I
 	CK(cudaEventRecord(ctx->t_begin, ctx->st));
 	CK(cudaMemcpyAsync(d0, I0, sizeof(float) * plane * n, cudaMemcpyDefault, ctx->st));
 	CK(cudaMemcpyAsync(d1, I1, sizeof(float) * plane * n, cudaMemcpyDefault, ctx->st));
-	int *d_timed_out = nullptr, timed_out = 0;
+	int *d_timed_out = nullptr;
 	bm4dof_status s = tvl1_run(ctx, d0, d1, W, H, n, false, p, du, dv, &d_timed_out);
 	if (s != BM4DOF_OK) return s;
 	// [pair][2][y][x]
@@ -1909,11 +1912,10 @@ bm4dof_status bm4dof_tvl1_pairs(bm4dof_ctx *ctx, const float *I0, const float *I
 	                     cudaMemcpyDeviceToDevice, ctx->st));
 	const size_t in_bytes = sizeof(float) * plane * n, uv_bytes = 2 * in_bytes;
 	if (!overlap(uv, uv_bytes, I0, in_bytes) && !overlap(uv, uv_bytes, I1, in_bytes)) map_output(uv, uv_bytes);
+	if ((s = tvl1_wait(ctx, d_timed_out)) != BM4DOF_OK) return s;
 	CK(cudaMemcpyAsync(uv, duv, sizeof(float) * plane * 2 * n, cudaMemcpyDefault, ctx->st));
-	CK(cudaMemcpyAsync(&timed_out, d_timed_out, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
 	CK(cudaEventRecord(ctx->t_end, ctx->st));
 	CK(cudaStreamSynchronize(ctx->st));
-	if (timed_out) return tvl1_timed_out();
 	for (int k = 0; k < 5; k++) ctx->ms[k] = 0.f;
 	cudaEventElapsedTime(&ctx->ms[4], ctx->t_begin, ctx->t_end);
 	return BM4DOF_OK;
@@ -1948,7 +1950,7 @@ bm4dof_status bm4dof_tvl1_video(bm4dof_ctx *ctx, const float *video, unsigned W,
 	CK(cudaEventRecord(ctx->t_begin, st));
 	CK(cudaMemcpyAsync(dvid, video, sizeof(float) * plane * F, cudaMemcpyDefault, st));
 	// pairs 0..F-2: t -> t+1 (forward); F-1..2F-3: t+1 -> t (backward of t+1)
-	int *d_timed_out = nullptr, timed_out = 0;
+	int *d_timed_out = nullptr;
 	bm4dof_status s = tvl1_run(ctx, dvid, dvid + plane, W, H, n, true, p, du, dv, &d_timed_out);
 	if (s != BM4DOF_OK) return s;
 	const size_t pb = sizeof(float) * plane;
@@ -1962,12 +1964,11 @@ bm4dof_status bm4dof_tvl1_video(bm4dof_ctx *ctx, const float *video, unsigned W,
 	CK(cudaMemcpyAsync(dbf, dbf + 2 * plane, 2 * pb, cudaMemcpyDeviceToDevice, st));
 	if (!overlap(fflow, 2 * pb * F, video, pb * F)) map_output(fflow, 2 * pb * F);
 	if (!overlap(bflow, 2 * pb * F, video, pb * F)) map_output(bflow, 2 * pb * F);
+	if ((s = tvl1_wait(ctx, d_timed_out)) != BM4DOF_OK) return s;
 	CK(cudaMemcpyAsync(fflow, dff, 2 * pb * F, cudaMemcpyDefault, st));
 	CK(cudaMemcpyAsync(bflow, dbf, 2 * pb * F, cudaMemcpyDefault, st));
-	CK(cudaMemcpyAsync(&timed_out, d_timed_out, sizeof(int), cudaMemcpyDeviceToHost, st));
 	CK(cudaEventRecord(ctx->t_end, st));
 	CK(cudaStreamSynchronize(st));
-	if (timed_out) return tvl1_timed_out();
 	for (int k = 0; k < 5; k++) ctx->ms[k] = 0.f;
 	cudaEventElapsedTime(&ctx->ms[4], ctx->t_begin, ctx->t_end);
 	return BM4DOF_OK;
