@@ -38,6 +38,7 @@
 #include <string>
 #include <vector>
 
+#include "divide.hpp"
 #include "internal.hpp"
 
 namespace cg = cooperative_groups;
@@ -478,16 +479,6 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned *p)
 	unsigned v;
 	asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
 	return v;
-}
-
-// a / b with y = 1 / b correctly rounded: Markstein's theorem (IBM J. Res. Dev.
-// 34(1), 1990) makes q + r y the correctly rounded quotient while the remainder
-// r is exact
-__device__ __forceinline__ float divide_by(float a, float b, float y)
-{
-	if ((fabsf(a) < 0x1p-100f && a != 0.f) || b > 0x1p60f) return a / b;
-	const float q = a * y;
-	return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
 // All warping steps of one level for gridDim.x / tiles pairs, a block a tile of
