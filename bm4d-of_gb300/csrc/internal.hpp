@@ -168,7 +168,7 @@ struct LearnedArgs {
 	long long ga, gb;                    // group range (rows are g - ga)
 	const uint8_t *nsimp, *alive;
 	const uint32_t *idx;
-	const float *basis, *binv, *win;
+	const float *basis, *binv;
 	__nv_bfloat16 *feat;                 // features: [rows][80]
 	const float *gains;                  // apply: [rows][64], or null (no network)
 	float *vals, *wslot;                 // apply: aggregation terms, member weights

@@ -138,7 +138,7 @@ __device__ __forceinline__ float feature_of(float var, float sigma2)
 
 template <int NS, int MODE>
 __device__ void group_body(const LearnedArgs &a, const StepParams &sp, long long g, float *Gs, float *Zs,
-                           const float *Bs, const float *Bi, const float *win, float *red, int bar)
+                           const float *Bs, const float *Bi, float *red, int bar)
 {
 	const int k = threadIdx.x & (kSub - 1);   // coefficient (transform) / pixel (inverse)
 	const float sigma2 = sp.sigma * sp.sigma;
@@ -246,9 +246,8 @@ learned_kernel(LearnedArgs a, StepParams sp)
 	extern __shared__ __align__(16) float lsm[];
 	float *Bs = lsm;                    // Bs[p][k] = basis[k][p]
 	float *Bi = Bs + kSpc * kSpc;       // Bi[k][p] = binv[k][p]
-	float *win = Bi + kSpc * kSpc;
 	const int sub = threadIdx.x / kSub, k = threadIdx.x % kSub;
-	float *Gs = win + kSpc + sub * 2 * sp.np * kSpc;
+	float *Gs = Bi + kSpc * kSpc + sub * 2 * sp.np * kSpc;
 	float *Zs = Gs + sp.np * kSpc;
 	__shared__ int s_mx[kGroupsPerCta][kMaxNp], s_my[kGroupsPerCta][kMaxNp], s_mt[kGroupsPerCta][kMaxNp];
 	__shared__ float s_red[kGroupsPerCta][2];
@@ -257,7 +256,6 @@ learned_kernel(LearnedArgs a, StepParams sp)
 		Bs[p * kSpc + kk] = a.basis[i];
 		Bi[i] = a.binv[i];
 	}
-	for (int i = threadIdx.x; i < kSpc; i += blockDim.x) win[i] = a.win[i];
 	__syncthreads();
 	const int bar = 1 + sub;
 	const int px = sp.px;
@@ -282,12 +280,12 @@ learned_kernel(LearnedArgs a, StepParams sp)
 		}
 		sub_sync(bar);
 		switch (ns) {
-		case 1: group_body<1, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
-		case 2: group_body<2, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
-		case 4: group_body<4, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
-		case 8: group_body<8, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
-		case 16: group_body<16, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
-		default: group_body<32, MODE>(a, sp, g, Gs, Zs, Bs, Bi, win, s_red[sub], bar); break;
+		case 1: group_body<1, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
+		case 2: group_body<2, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
+		case 4: group_body<4, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
+		case 8: group_body<8, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
+		case 16: group_body<16, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
+		default: group_body<32, MODE>(a, sp, g, Gs, Zs, Bs, Bi, s_red[sub], bar); break;
 		}
 		sub_sync(bar);
 	}
@@ -614,7 +612,7 @@ cudaError_t launch_tc(const LearnedArgs &a, const StepParams &sp, int nsm, cudaS
 template <int MODE>
 cudaError_t launch_mode(const LearnedArgs &a, const StepParams &sp, int nsm, cudaStream_t st)
 {
-	const size_t smem = sizeof(float) * (2 * kSpc * kSpc + kSpc + (size_t)kGroupsPerCta * 2 * sp.np * kSpc);
+	const size_t smem = sizeof(float) * (2 * kSpc * kSpc + (size_t)kGroupsPerCta * 2 * sp.np * kSpc);
 	cudaError_t e = cudaFuncSetAttribute(learned_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess) return e;
 	int per_sm = 0;

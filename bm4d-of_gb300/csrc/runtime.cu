@@ -732,7 +732,6 @@ bm4dof_status launch_step(bm4dof_ctx *ctx, int slot, const Image &noisy, const I
 	la.idx = S.d_idx;
 	la.basis = S.d_basis;
 	la.binv = S.d_binv;
-	la.win = S.d_win;
 	la.kappa = ctx->kappa;
 	la.nfallback = S.d_small + 3;
 	if (mode.samples) {

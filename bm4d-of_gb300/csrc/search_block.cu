@@ -45,7 +45,6 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
-#include <cstdlib>
 
 #include "common.cuh"
 #include "internal.hpp"
@@ -224,8 +223,6 @@ struct BlockArgs {
 	unsigned *gcount;
 	float eps;                         // relative error bound between two sums of one distance
 };
-
-__device__ __forceinline__ unsigned redux_min(unsigned v) { return __reduce_min_sync(0xffffffffu, v); }
 
 // Whether a block of `rounds` rounds of 32 columns is cheaper here than four
 // groups with `cand` candidates in all in search.cu's kernel.  Nanoseconds of the
