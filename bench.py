@@ -48,9 +48,9 @@ WORKLOADS = {
 CLI = dict(px1=4, px2=4, pt1=4, pt2=4, wx1=21, wx2=21, np1=16, np2=16, b1=3.0)
 METRIC = "megapixel-frames/s at 1 GPU, plain vs learned/mixed at ≤0.05 dB PSNR loss"
 UNIT = "MPF/s"
-# ncu dram__bytes_read + dram__bytes_write of one step-1 search_block_kernel
-# launch on 480x272x12 (one --set full capture of the small workload)
-SEARCH_TRAFFIC_SMALL = 12.15e6 + 0.18e6
+# ncu dram__bytes_read + dram__bytes_write of a search_block_kernel launch on
+# 480x272x12, mean of step 1 and step 2 (one --set full capture of the small workload)
+SEARCH_TRAFFIC_SMALL = ((12.2e6 + 0.2e6) + 17.2e6) / 2
 # CPU sample (crop of the same workload) for the host-core baseline: 12
 # frames, so that every reference patch has the full 9-frame search range it
 # has in the long video
@@ -440,17 +440,17 @@ def main():
     if rank != 0:
         return 0
     # roofline of the dominant kernel (patch search by 2x2 blocks of groups): FP32
-    # lane operations -- 36 squared differences (a subtraction and a multiply-add)
-    # per patch frame and candidate serve four groups -- over the measured launch
-    # duration
+    # lane operations -- (4 + step)^2 squared differences (a subtraction and a
+    # multiply-add) per patch frame and candidate serve four groups, step the
+    # reference grid's -- over the measured launch duration
     whf = W * H * F
     groups = [round(r * whf / 100.0) for r in ratios]
     ncand = 21 * 21 * 9
-    flops_per_launch = statistics.mean(g * 2 * 36 * 4 / 4 * ncand for g in groups)
+    flops_per_launch = statistics.mean(g * 2 * (4 + p.offSet) ** 2 * 4 / 4 * ncand for g, p in zip(groups, (p1, p2)))
     launch_ms = statistics.mean(searches) / 2.0
     achieved = flops_per_launch / (launch_ms / 1e3) / 1e12
-    # the search's instruction mix timed alone on this GPU (registers only,
-    # packed subtract and multiply, scalar adds): the rate it could reach
+    # the search's instruction mix timed alone on this GPU (registers only, packed
+    # subtract and multiply-add): the rate it could reach
     peak, mix_ms = bm4dof.fp32_mix_rate(local)
     nominal = 152 * 128 * 2.07e9 / 1e12
     psnr = lambda a, b: float(10 * np.log10(255.0 ** 2 / np.mean((a.astype(np.float64) - b) ** 2)))
@@ -463,15 +463,15 @@ def main():
         "config": config(args),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
-                     # DRAM bytes per launch: ncu capture of the 480x272x12 step-1 launch
-                     # (12.15 MB read + 0.18 MB written), scaled by the pixel count
+                     # DRAM bytes per launch: ncu capture of the 480x272x12 launches
+                     # (12.4 MB in step 1, 17.2 in step 2), scaled by the pixel count
                      "traffic": SEARCH_TRAFFIC_SMALL * (W * H * F) / (480 * 272 * 12),
                      "traffic_source": "ncu dram__bytes_read+write of search_block_kernel on 480x272x12, "
                                        "scaled by pixels (the frames and flows, read about once)",
                      "kernel": "search_block_kernel",
-                     "peak_source": "measured on this GPU by bm4dof_fp32_mix_rate: the per-group search's FP32 "
-                                    "instruction mix (packed sub/mul.rn.f32x2 + scalar adds) from registers, "
-                                    "3 ops per element (MEASURED_PEAKS.json has HBM and bf16 tensor peaks only)",
+                     "peak_source": "measured on this GPU by bm4dof_fp32_mix_rate: the block search's FP32 "
+                                    "instruction mix (packed sub and fma.rn.f32x2) from registers, "
+                                    "2 ops per difference (MEASURED_PEAKS.json has HBM and bf16 tensor peaks only)",
                      "nominal_fp32_tops": nominal, "frac_of_nominal": achieved / nominal},
         "e2e": {"value": e2e_value, "unit": UNIT,
                 "h2d_bytes_per_step": int(nz.nbytes + ff.nbytes + bf.nbytes),

@@ -620,7 +620,7 @@ def tc_selftest(a, b):
 
 
 def fp32_mix_rate(device=0):
-    """Measured FP32 rate (tera-operations/s, 3 per patch element) of the exact
+    """Measured FP32 rate (tera-operations/s, 2 per squared difference) of the exact
     search's instruction mix (bm4dof_fp32_mix_rate) and one launch's ms."""
     t, ms = C.c_float(), C.c_float()
     _check(load().bm4dof_fp32_mix_rate(device, C.byref(t), C.byref(ms)))

@@ -1,20 +1,17 @@
 // peaks.cu -- measured FP32 rate of the exact search's instruction mix, the
 // denominator of that kernel's roofline.
 //
-// The exact distance (nldct.cpp:1261-1274) is one rounded subtract, multiply
-// and add per patch element, no FMA.  The search issues them as one packed
-// subtract and one packed multiply per two elements (sub/mul.rn.f32x2) and
-// two scalar adds (search_common.cuh, sqdiff2); the GPU's nominal FP32 rate
-// (one operation per lane and clock) says nothing about how fast that mix
-// issues.  fp32_mix_kernel runs the same mix from registers only, with eight
-// independent chains per thread and 64 warps per SM, and counts 3 operations
-// per element, the unit of the search's algorithmic work.
+// The search by blocks (search_block.cu) forms a squared difference with a subtract
+// and a multiply-add, two differences to a packed instruction (f32x2); the GPU's
+// nominal FP32 rate (one operation per lane and clock) says nothing about how fast
+// that mix issues.  fp32_mix_kernel runs it from registers only, with eight
+// independent chains per thread and 64 warps per SM, and counts 2 operations per
+// difference, the unit of the search's work.
 #include <cuda_runtime.h>
 #include <cstdint>
 
 #include "../../include/bm4dof.h"
 #include "internal.hpp"
-#include "search_common.cuh"
 
 namespace bm4dof {
 
@@ -25,24 +22,22 @@ constexpr int kMixThreads = 256;
 
 __global__ void __launch_bounds__(kMixThreads) fp32_mix_kernel(float *out, int iters, float seed)
 {
-	float acc[kChains], ref[kChains];
+	float2 acc[kChains], ref[kChains];
 #pragma unroll
 	for (int j = 0; j < kChains; j++) {
-		acc[j] = seed * (float)(threadIdx.x + j);
-		ref[j] = seed + (float)j;
+		acc[j] = make_float2(seed * (float)(threadIdx.x + j), seed * (float)j);
+		ref[j] = make_float2(seed + (float)j, seed - (float)j);
 	}
 	for (int i = 0; i < iters; i++) {
 #pragma unroll
 		for (int j = 0; j < kChains; j++) {
-			// two elements: (ref - acc)^2 and (ref + 1 - acc)^2, added in order
-			float m0, m1;
-			sqdiff2(ref[j], ref[j] + 1.f, acc[j], acc[j], m0, m1);
-			acc[j] = __fadd_rn(__fadd_rn(acc[j], m0), m1);
+			const float2 d = __fadd2_rn(ref[j], acc[j]);
+			acc[j] = __ffma2_rn(d, d, acc[j]);
 		}
 	}
 	float s = 0.f;
 #pragma unroll
-	for (int j = 0; j < kChains; j++) s += acc[j];
+	for (int j = 0; j < kChains; j++) s += acc[j].x + acc[j].y;
 	if (s == 1.2345f) out[blockIdx.x] = s;   // keeps the chains live, never true in practice
 }
 
@@ -88,8 +83,8 @@ extern "C" bm4dof_status bm4dof_fp32_mix_rate(int device, float *tops, float *ms
 		set_error(std::string("bm4dof_fp32_mix_rate: ") + cudaGetErrorString(e));
 		return BM4DOF_ERR_CUDA;
 	}
-	// per chain and iteration: two elements, 3 operations each
-	const double ops = 4.0 * blocks * (double)kMixThreads * iters * kChains * 6.0;
+	// per chain and iteration: two differences, 2 operations each
+	const double ops = 4.0 * blocks * (double)kMixThreads * iters * kChains * 4.0;
 	*tops = (float)(ops / (t * 1e-3) / 1e12);
 	if (ms) *ms = t / 4.f;
 	return BM4DOF_OK;

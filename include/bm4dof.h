@@ -389,10 +389,10 @@ bm4dof_status bm4dof_mixed_stats(bm4dof_ctx *ctx, unsigned long long *groups, un
                                  unsigned long long *uncertified);
 
 /* No counterpart in the reference: the measured FP32 rate of the exact patch
- * search's instruction mix on `device` (per two patch elements one packed
- * subtract, one packed multiply and two scalar adds, the reference's
- * separately rounded operations), in tera-operations per second counting 3
- * per element -- the denominator of that kernel's roofline.  *ms (may be
+ * search's instruction mix on `device` (the search by blocks: per two squared
+ * differences one packed subtract and one packed multiply-add), in
+ * tera-operations per second counting 2 per difference -- the denominator of
+ * that kernel's roofline.  *ms (may be
  * NULL) receives one launch's time.  Allocates a few bytes; synchronises. */
 bm4dof_status bm4dof_fp32_mix_rate(int device, float *tops, float *ms);
 
