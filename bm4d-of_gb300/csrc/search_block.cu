@@ -27,7 +27,7 @@
 //     overflows and sources with values that are not finite.
 //   * Blocks that do not pay.  The four windows of a block follow their own
 //     flows; where those differ the block covers the windows' union, which may
-//     cost more than the four windows one by one (pays_off).  And in a block of
+//     cost more than the four windows one by one (Cost).  And in a block of
 //     one value every group finds itself and its neighbours at distance 0, a tie.
 //     Such blocks are left to search.cu's kernel before they are computed: flat
 //     854x480x8, 4x4x4, both steps, 40.1 ms with them computed, 31.8 without.
@@ -224,21 +224,22 @@ struct BlockArgs {
 	float eps;                         // relative error bound between two sums of one distance
 };
 
-// Whether a block of `rounds` rounds of 32 columns is cheaper here than four
-// groups with `cand` candidates in all in search.cu's kernel.  Nanoseconds of the
-// whole GPU, fitted to both kernels' times (854x480x8, windows of 9, 21 and 39; 8x8
-// and 7x7 also 7x7 windows): a block takes 13 and 0.025 (4x4x4) or 0.036 a round
-// and pixel of the block, a group 10 (4x4x4) or 50 and 0.011 a candidate and
-// channel.  4x4x4, step 2, 21x21 windows over 5 frames: 49 against 137, so the
-// rounds may rise from 10 to 34.  Without the rule flows with a noise of 8 / 20
+// What a frame's share of a block costs here more than its four patches' candidates
+// cost in search.cu's kernel; a block whose frames cost more than kSpare together is
+// cheaper there.  In 1/1024 nanoseconds of the whole GPU and per channel, fitted to
+// both kernels' times (854x480x8, windows of 9, 21 and 39; 8x8 and 7x7 also 7x7
+// windows): a block takes 13 ns and, for every 32 columns of displacements, 0.025
+// (4x4x4) or 0.036 a pixel of the block; a group 10 (4x4x4) or 50 and 0.011 a
+// candidate.  4x4x4, step 2, 21x21 windows over 5 frames: 49 against 137 ns, so the
+// columns may rise from 315 to 1090.  Without the rule flows with a noise of 8 / 20
 // pixels took 21.9 / 52.2 ms (480x272x10, both steps) where the per-group kernel
 // takes 15.0 / 16.0.
 template <int P, int S, int PT>
-__device__ __forceinline__ bool pays_off(int rounds, int cand, int chn)
-{
-	constexpr float kRound = (P == 4 ? 0.025f : 0.036f) * PT * (P + S) * (P + S), kGroup = P == 4 ? 10.f : 50.f;
-	return 13.f + kRound * (float)(rounds * chn) <= 4.f * kGroup + 0.011f * (float)(cand * chn);
-}
+struct Cost {
+	static constexpr int kColumn = (int)((P == 4 ? 0.025f : 0.036f) * PT * (P + S) * (P + S) * 32.f + 0.5f);
+	static constexpr int kCandidate = 11;
+	static constexpr int kSpare = (P == 4 ? 4 * 10 - 13 : 4 * 50 - 13) * 1024;
+};
 
 constexpr float kTiny = 1e-35f;        // below this the products may underflow
 constexpr float kMaxFinite = 3.0e38f;
@@ -377,8 +378,9 @@ search_block_kernel(Image src, StepParams sp, BlockArgs a)
 #pragma unroll
 		for (int k = 0; k < 4; k++) K[k] = min(sp.np, __reduce_add_sync(0xffffffffu, cand[k]));
 		// (in one condition with the next: another exit here costs the main loop registers)
-		wide |= !pays_off<P, S, PT>((nitems + 31) / 32, __reduce_add_sync(0xffffffffu, cand[0] + cand[1] + cand[2] + cand[3]) *
-		                                                (4 / (__popc(have) * __popc(havey))), chn);
+		using Co = Cost<P, S, PT>;
+		const int four = (cand[0] + cand[1] + cand[2] + cand[3]) << ((px2 ? 0 : 1) + (py2 ? 0 : 1));
+		wide |= __reduce_add_sync(0xffffffffu, items * Co::kColumn - four * Co::kCandidate) * chn > Co::kSpare;
 		// ---- reference pixels: per row S pairs (left, right), then the middle --
 		// (not unrolled: 54.5 -> 53.9 ms on 854x480x20, both steps)
 		bool flat = true;
