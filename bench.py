@@ -50,7 +50,7 @@ METRIC = "megapixel-frames/s at 1 GPU, plain vs learned/mixed at ≤0.05 dB PSNR
 UNIT = "MPF/s"
 # ncu dram__bytes_read + dram__bytes_write of a search_block_kernel launch on
 # 480x272x12, mean of step 1 and step 2 (one --set full capture of the small workload)
-SEARCH_TRAFFIC_SMALL = ((12.2e6 + 0.2e6) + 17.2e6) / 2
+SEARCH_TRAFFIC_SMALL = ((12.86e6 + 0.31e6) + (17.77e6 + 0.14e6)) / 2
 # CPU sample (crop of the same workload) for the host-core baseline: 12
 # frames, so that every reference patch has the full 9-frame search range it
 # has in the long video
@@ -464,7 +464,7 @@ def main():
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
                      # DRAM bytes per launch: ncu capture of the 480x272x12 launches
-                     # (12.4 MB in step 1, 17.2 in step 2), scaled by the pixel count
+                     # (13.2 MB in step 1, 17.9 in step 2), scaled by the pixel count
                      "traffic": SEARCH_TRAFFIC_SMALL * (W * H * F) / (480 * 272 * 12),
                      "traffic_source": "ncu dram__bytes_read+write of search_block_kernel on 480x272x12, "
                                        "scaled by pixels (the frames and flows, read about once)",
